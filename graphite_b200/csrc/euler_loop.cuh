@@ -1,0 +1,68 @@
+// Arguments and launch of the persistent Euler loop (euler_loop.cu).
+#pragma once
+
+#include "euler_ops.cuh"
+
+namespace gb {
+
+// One cell per thread.  Up to kLoopWide threads per block a thread may use
+// 128 registers and keeps its own face states and ghosts in shared memory.
+constexpr int kLoopWide = 256;
+constexpr int kLoopFull = 416;          // all of a cell's geometry in shared memory up to here
+constexpr int kLoopMax = 512;
+constexpr int kLoopBlocksPerSM = 2;
+constexpr int kLoopSmem = 112 * 1024;   // dynamic shared memory of a block, at most
+
+// 16 bytes that are written and read as one: three words and the tag that
+// says which iteration they belong to.
+struct alignas(16) TagRec {
+    uint32_t x, y, z, tag;
+};
+
+struct LoopVerdict {
+    unsigned int count;     // tag of the last iteration that has been judged
+    unsigned int halt;
+};
+
+struct EulerLoopArgs {
+    MeshDev m;
+    const float4* ghost_off;              // per ghost: its face centre - its centroid
+    float* rho[2];
+    float4* rhou[2];
+    float* rhoe[2];
+    float* rec_rho;
+    float4* rec_rhou;
+    float* err;
+    GhostBcTable ghosts;
+    float cfl;
+    int iters, cur0;
+    double tol;
+    RunCtl* ctl;
+    double *hist, *hist_rho;              // hist_rho null: the density part is not summed
+    unsigned long long hist_cap;
+    double *out, *partials;               // the residual, and its sums by 256-cell group
+    int n_groups, n_blocks;
+    unsigned int tag0;                    // tags of this launch: tag0 + iteration
+    TagRec* state[2];                     // 2 per cell and buffer: (rho, u, v), (w, E)
+    TagRec* rec;                          // 2 per entry: (rho, u, v), (w, E)
+    TagRec *wsum, *wsum_rho;              // per warp: a double
+    unsigned long long* verdict;          // LoopVerdict
+};
+
+// shared memory of a block (bytes); lean: without the face normals and areas
+constexpr int loop_smem_of(int max_faces, int threads, bool lean) {
+    return threads * ((lean ? 28 : 44) * max_faces + 28 + (threads <= kLoopWide && !lean ? 64 + 28 * max_faces : 0));
+}
+constexpr bool loop_lean(int max_faces, int threads) {
+    return threads > kLoopFull || loop_smem_of(max_faces, threads, false) > kLoopSmem;
+}
+constexpr int loop_smem(int max_faces, int threads) {
+    return loop_smem_of(max_faces, threads, loop_lean(max_faces, threads));
+}
+
+void launch_ghost_off(const DevMesh& d, float4* ghost_off, cudaStream_t s);
+cudaError_t launch_euler_loop(EulerLoopArgs& a, int max_faces, int threads, bool transposed, cudaStream_t s);
+
+MeshDev mesh_dev(const DevMesh& m);
+
+}  // namespace gb

@@ -70,7 +70,7 @@ struct RunCtl {
     unsigned long long it_run;     // iterations run since the loop started
     double res0;
     int halt;
-    int pad;
+    int error;                     // nonzero: a wait of the persistent loop gave up
 };
 
 // Pointers of the three conserved fields as one kernel argument.

@@ -272,6 +272,8 @@ int gbApplyBoundaryConditions(cuMesh* mesh);
 
 /* Runs n_iter iterations of the PhysicsEuler::step loop (boundary conditions
  * in the given order, prepare, step, residual sum) as a replayed CUDA graph,
+ * or, on meshes that fit on the GPU one cell per thread (about 150,000 cells),
+ * as one persistent cooperative launch per check_every iterations,
  * writing the residual sum of each iteration to residual_history (host
  * array of n_iter doubles, may be NULL).  With tolerance > 0 it stops after
  * the first iteration in which residual/residual[0] < tolerance: the device
@@ -286,7 +288,9 @@ int gbApplyBoundaryConditions(cuMesh* mesh);
  * gradients and limiters of the fields are not stored (the per-call
  * FvmEulerStepPrepare stores them).  Inside, all conditions are applied by
  * one ghost kernel, or, when the ghosts number at least a quarter of the
- * cells, by the gradient kernel itself. */
+ * cells and in the persistent launch, by the gradient pass itself.  The
+ * persistent launch waits on the GPU for its own cells' data; a wait that
+ * gives up (after some seconds) ends the call with an error. */
 int64_t gbEulerRun(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* rhoe, FvmField* error,
                    gb_scalar cfl, int64_t n_iter, const gbBc* bcs, int n_bc, double tolerance,
                    int check_every, double* residual_history);
