@@ -133,6 +133,7 @@ struct MeshImpl {
     PendingBcs pending;
     RunGraphs euler_run, nsi_run;
     LoopPlan loop;
+    Workspace ws;
     cudaStream_t capture = nullptr;   // stream the loops are captured on
     double* h_result = nullptr;       // pinned: FvmFieldReduceSum's value on the host
 };
@@ -784,6 +785,22 @@ int64_t run_loop(MeshImpl* mi, EulerLoopArgs& a, bool transposed, int& cur, int6
 }
 }  // namespace
 
+bool Workspace::ensure(size_t bytes, const char* what) {
+    if (!host && !cuda_ok(cudaMallocHost((void**)&host, kHostWords * sizeof(double)), what)) return false;
+    if (dev_bytes >= bytes) return true;
+    if (dev) cudaFree(dev);
+    dev = nullptr;
+    dev_bytes = 0;
+    if (!cuda_ok(cudaMalloc(&dev, bytes), what)) return false;
+    dev_bytes = bytes;
+    return true;
+}
+
+Workspace::~Workspace() {
+    if (dev) cudaFree(dev);
+    if (host) cudaFreeHost(host);
+}
+
 bool mesh_access(cuMesh* mesh, MeshAccess* out) {
     MeshImpl* mi = impl(mesh);
     if (!mi) { set_error("null mesh"); return false; }
@@ -795,6 +812,7 @@ bool mesh_access(cuMesh* mesh, MeshAccess* out) {
     out->G = mi->topo.G;
     out->topo = &mi->topo;
     out->num = &mi->num;
+    out->ws = &mi->ws;
     return true;
 }
 
@@ -1010,9 +1028,10 @@ int FvmEulerInit(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* rhoe, gb
     const float3 ru = make_float3(vel.x * r, vel.y * r, vel.z * r);
     const float e = pressure / 0.4f + 0.5f * r * (vel.x * vel.x + vel.y * vel.y + vel.z * vel.z);
     const int64_t n = (int64_t)impl(rho)->size;
-    for (int k = 0; k < 2; ++k)
-        launch_init(n, (float*)impl(rho)->val[k], (float4*)impl(rhou)->val[k], (float*)impl(rhoe)->val[k], r, ru, e,
-                    t_stream);
+    float* const pr[2] = {(float*)impl(rho)->val[0], (float*)impl(rho)->val[1]};
+    float4* const pu[2] = {(float4*)impl(rhou)->val[0], (float4*)impl(rhou)->val[1]};
+    float* const pe[2] = {(float*)impl(rhoe)->val[0], (float*)impl(rhoe)->val[1]};
+    launch_init(n, pr, pu, pe, r, ru, e, t_stream);
     impl(rho)->cur = impl(rhou)->cur = impl(rhoe)->cur = 0;
     return launch_ok("FvmEulerInit") ? 0 : 1;
 }
@@ -1525,21 +1544,18 @@ int gbNSIWallForce(cuMesh* mesh, FvmField* velocity, FvmField* pressure, unsigne
     force[0] = force[1] = force[2] = 0.0;
     if (g1 <= g0) return 0;
     const int blocks = (int)((g1 - g0 + kBlock - 1) / kBlock);
-    double* d = nullptr;
-    if (!dalloc(d, (size_t)3 * blocks + 3, "gbNSIWallForce")) return 1;
+    std::lock_guard<std::mutex> lock(mi->ws.mu);
+    if (!mi->ws.ensure((size_t)3 * blocks * sizeof(double), "gbNSIWallForce")) return 1;
     const int cur = impl(pressure)->cur;
     cudaStream_t s = t_stream;
     // the gradient of the current state (the one stored may be a step old)
     launch_nsi_grad(mi->dev, (const float*)impl(pressure)->val[cur], (const float4*)impl(velocity)->val[cur],
                     impl(pressure)->grad, impl(velocity)->grad, t_nsi.limited, s);
     launch_nsi_force(mi->dev, g0, g1, (const float*)impl(pressure)->val[cur], (const float4*)impl(velocity)->val[cur],
-                     impl(velocity)->grad, (float)t_nsi.viscosity, t_nsi.corrected, t_nsi.density, d, d + 3 * blocks,
-                     s);
-    const bool ok = launch_ok("gbNSIWallForce") &&
-                    cuda_ok(cudaMemcpyAsync(force, d + 3 * blocks, 3 * sizeof(double), cudaMemcpyDeviceToHost, s),
-                            "gbNSIWallForce") &&
-                    cuda_ok(cudaStreamSynchronize(s), "gbNSIWallForce");
-    dfree(d);
+                     impl(velocity)->grad, (float)t_nsi.viscosity, t_nsi.corrected, t_nsi.density,
+                     (double*)mi->ws.dev, mi->ws.host, s);
+    const bool ok = launch_ok("gbNSIWallForce") && cuda_ok(cudaStreamSynchronize(s), "gbNSIWallForce");
+    if (ok) memcpy(force, mi->ws.host, 3 * sizeof(double));
     return ok ? 0 : 1;
 }
 

@@ -27,6 +27,7 @@ namespace gb {
 namespace {
 
 constexpr int kMaxRegions = 16;
+constexpr size_t kHistKeep = 8u << 20;    // values of residual history a batch keeps room for (64 MB)
 
 struct InstDev {
     float* rho[2];
@@ -456,7 +457,15 @@ struct gbBatchImpl {
     int schedule = 1;     // 0 instance-major, 1 tile-major
     int variant = 0;      // register budget of the gradient/flux kernels
     int2* d_cell_items = nullptr;
-    int n_cell_items = 0;
+    int n_cell_items = 0, items_cap = 0;
+    std::vector<int> items_key;
+    cudaStream_t capture = nullptr;           // stream and graph of the replayed iteration, and what the graph bakes in
+    cudaGraphExec_t exec = nullptr;
+    std::vector<double> exec_key;
+    double* d_hist = nullptr;                 // residual histories of a run, kept up to kHistKeep values
+    size_t hist_cap = 0;
+    gb::Workspace ws;
+    bool table_stale = false;                 // d_inst is ahead of h_inst
     gb::GridSync* d_sync = nullptr;   // barrier and work counters of the persistent kernel
     bool inject_barrier_fault = false;
     std::vector<void*> allocations;
@@ -493,6 +502,10 @@ int64_t tiles_of(const Batch* b, int inst, int tile) {
 }
 
 bool build_items(Batch* b) {
+    std::vector<int> key = {b->tile, b->schedule};   // what the list depends on
+    for (const InstDev& I : b->h_inst) key.push_back(I.status == 0);
+    if (b->d_cell_items && b->items_key == key) return true;
+    b->items_key.clear();
     std::vector<int2> items;
     auto active = [&](int i) { return b->h_inst[i].status == 0; };
     if (b->schedule == 0) {
@@ -512,14 +525,21 @@ bool build_items(Batch* b) {
                 for (int i : insts) items.push_back(make_int2(i, (int)t));
         }
     }
-    if (b->d_cell_items) cudaFree(b->d_cell_items);
-    b->d_cell_items = nullptr;
     b->n_cell_items = (int)items.size();
-    if (!ok_(cudaMalloc((void**)&b->d_cell_items, std::max<size_t>(items.size(), 1) * sizeof(int2)), "batch items"))
-        return false;
+    if (b->items_cap < b->n_cell_items || !b->d_cell_items) {
+        if (b->d_cell_items) cudaFree(b->d_cell_items);
+        b->d_cell_items = nullptr;
+        b->items_cap = 0;
+        const size_t cap = std::max<size_t>(items.size(), 1);
+        if (!ok_(cudaMalloc((void**)&b->d_cell_items, cap * sizeof(int2)), "batch items")) return false;
+        b->items_cap = (int)cap;
+    }
     cudaStream_t s = (cudaStream_t)gbGetStream();
-    return ok_(cudaMemcpyAsync(b->d_cell_items, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice, s),
-               "batch items");
+    if (!ok_(cudaMemcpyAsync(b->d_cell_items, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice, s),
+             "batch items"))
+        return false;
+    b->items_key = key;
+    return true;
 }
 
 // partial-sum buffers sized for the current tile
@@ -537,17 +557,24 @@ bool size_partials(Batch* b) {
 }
 
 bool upload_inst(Batch* b) {
+    b->table_stale = false;
     return ok_(cudaMemcpyAsync(b->d_inst, b->h_inst.data(), b->h_inst.size() * sizeof(InstDev), cudaMemcpyHostToDevice,
                                (cudaStream_t)gbGetStream()),
                "batch table");
 }
 
+// h_inst up to date with what the kernels of a run made of the table
+// (synchronises the stream when there is anything to fetch).
 bool download_inst(Batch* b) {
+    if (!b->table_stale) return true;
     cudaStream_t s = (cudaStream_t)gbGetStream();
-    return ok_(cudaMemcpyAsync(b->h_inst.data(), b->d_inst, b->h_inst.size() * sizeof(InstDev), cudaMemcpyDeviceToHost,
-                               s),
-               "batch table") &&
-           ok_(cudaStreamSynchronize(s), "batch table");
+    if (!ok_(cudaMemcpyAsync(b->h_inst.data(), b->d_inst, b->h_inst.size() * sizeof(InstDev), cudaMemcpyDeviceToHost,
+                             s),
+             "batch table") ||
+        !ok_(cudaStreamSynchronize(s), "batch table"))
+        return false;
+    b->table_stale = false;
+    return true;
 }
 
 // One cooperative launch of the persistent kernel for `iters` iterations of
@@ -653,20 +680,23 @@ int active_tile(const Batch* b, int tuned) {
 // the residual's float64 block sums are then taken over smaller blocks.
 int64_t run_loop(Batch* b, float cfl, int64_t max_iter, double tol, int check_every) {
     cudaStream_t s = (cudaStream_t)gbGetStream();
-    cudaStream_t cap = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    bool ok = ok_(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking), "batch graph");
+    bool ok = b->capture || ok_(cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking), "batch graph");
     auto capture = [&]() {
-        if (exec) cudaGraphExecDestroy(exec);
-        exec = nullptr;
+        // everything the captured launches bake in; the graph of an earlier run is replayed when it matches
+        const std::vector<double> key = {(double)(uintptr_t)b->d_cell_items, (double)b->n_cell_items, (double)b->tile,
+                                         (double)b->variant, (double)reference_momentum(), (double)cfl, tol};
+        if (b->exec && b->exec_key == key) return true;
+        if (b->exec) cudaGraphExecDestroy(b->exec);
+        b->exec = nullptr;
         cudaGraph_t graph = nullptr;
-        bool good = ok_(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal), "batch graph");
+        bool good = ok_(cudaStreamBeginCapture(b->capture, cudaStreamCaptureModeThreadLocal), "batch graph");
         if (good) {
-            enqueue_iteration(b, cfl, tol, cap);
-            good = ok_(cudaStreamEndCapture(cap, &graph), "batch graph") &&
-                   ok_(cudaGraphInstantiate(&exec, graph, 0), "batch graph");
+            enqueue_iteration(b, cfl, tol, b->capture);
+            good = ok_(cudaStreamEndCapture(b->capture, &graph), "batch graph") &&
+                   ok_(cudaGraphInstantiate(&b->exec, graph, 0), "batch graph");
         }
         if (graph) cudaGraphDestroy(graph);
+        b->exec_key = key;
         return good;
     };
     const bool persistent = b->variant >= kPersistentVariant;
@@ -676,12 +706,13 @@ int64_t run_loop(Batch* b, float cfl, int64_t max_iter, double tol, int check_ev
     int active = b->n_inst;
     while (ok && done < max_iter) {
         const int64_t chunk = std::min<int64_t>(check_every, max_iter - done);
+        b->table_stale = true;
         if (persistent) {
             ok = launch_persistent(b, cfl, tol, (int)chunk, s) && persistent_ok(b, s);
         } else {
             const int per_iter = 1 + (b->n_cell_items ? 2 : 0);
             for (int64_t i = 0; i < chunk && ok; ++i) {
-                ok = ok_(cudaGraphLaunch(exec, s), "batch graph launch");
+                ok = ok_(cudaGraphLaunch(b->exec, s), "batch graph launch");
                 count_launch(per_iter);
             }
         }
@@ -700,8 +731,6 @@ int64_t run_loop(Batch* b, float cfl, int64_t max_iter, double tol, int check_ev
             ok = ok && build_items(b) && ok_(cudaStreamSynchronize(s), "batch items") && (persistent || capture());
         }
     }
-    if (exec) cudaGraphExecDestroy(exec);
-    if (cap) cudaStreamDestroy(cap);
     if (ok && b->tile != tuned) {        // nothing is in flight: download_inst synchronised
         b->tile = tuned;
         ok = size_partials(b) && upload_inst(b) && ok_(cudaStreamSynchronize(s), "batch table");
@@ -810,6 +839,9 @@ void gbBatchFree(gbBatch* b) {
     if (!b) return;
     for (void* p : b->allocations) cudaFree(p);
     if (b->d_cell_items) cudaFree(b->d_cell_items);
+    if (b->d_hist) cudaFree(b->d_hist);
+    if (b->exec) cudaGraphExecDestroy(b->exec);
+    if (b->capture) cudaStreamDestroy(b->capture);
     delete b;
 }
 
@@ -823,9 +855,8 @@ int gbBatchInitUniform(gbBatch* b, int inst, gb_vector mach, gb_scalar pressure,
     const float c = sqrtf(1.4f * pressure / r);
     const float3 vel = make_float3(mach.x * c, mach.y * c, mach.z * c);
     const float e = pressure / 0.4f + 0.5f * r * (vel.x * vel.x + vel.y * vel.y + vel.z * vel.z);
-    for (int k = 0; k < 2; ++k)
-        launch_init(A.N + A.G, I.rho[k], I.rhou[k], I.rhoe[k], r, make_float3(vel.x * r, vel.y * r, vel.z * r), e,
-                    (cudaStream_t)gbGetStream());
+    launch_init(A.N + A.G, I.rho, I.rhou, I.rhoe, r, make_float3(vel.x * r, vel.y * r, vel.z * r), e,
+                (cudaStream_t)gbGetStream());
     return ok_(cudaGetLastError(), "gbBatchInitUniform") ? 0 : 1;
 }
 
@@ -836,18 +867,14 @@ int gbBatchSetState(gbBatch* b, int inst, const float* rho, const float* rhou, c
     const MeshAccess& A = b->acc[I.mesh];
     const int64_t NG = A.N + A.G;
     cudaStream_t s = (cudaStream_t)gbGetStream();
-    float* stage = nullptr;
-    if (!ok_(cudaMalloc((void**)&stage, NG * 5 * sizeof(float)), "gbBatchSetState")) return 1;
+    std::lock_guard<std::mutex> lock(b->ws.mu);
+    if (!b->ws.ensure((size_t)NG * 5 * sizeof(float), "gbBatchSetState")) return 1;
+    float* stage = (float*)b->ws.dev;
     bool ok = ok_(cudaMemcpyAsync(stage, rho, NG * 4, cudaMemcpyHostToDevice, s), "gbBatchSetState") &&
               ok_(cudaMemcpyAsync(stage + NG, rhou, NG * 12, cudaMemcpyHostToDevice, s), "gbBatchSetState") &&
               ok_(cudaMemcpyAsync(stage + 4 * NG, rhoe, NG * 4, cudaMemcpyHostToDevice, s), "gbBatchSetState");
-    for (int k = 0; k < 2 && ok; ++k) {
-        launch_scatter_scalar(NG, stage, A.d_cell_new, I.rho[k], s);
-        launch_scatter_vector(NG, stage + NG, A.d_cell_new, I.rhou[k], s);
-        launch_scatter_scalar(NG, stage + 4 * NG, A.d_cell_new, I.rhoe[k], s);
-    }
-    ok = ok && ok_(cudaStreamSynchronize(s), "gbBatchSetState");
-    cudaFree(stage);
+    if (ok) launch_scatter_state(NG, stage, A.d_cell_new, I.rho, I.rhou, I.rhoe, s);
+    ok = ok_(cudaStreamSynchronize(s), "gbBatchSetState") && ok;
     return ok ? 0 : 1;
 }
 
@@ -859,17 +886,15 @@ int gbBatchGetState(gbBatch* b, int inst, float* rho, float* rhou, float* rhoe) 
     const MeshAccess& A = b->acc[I.mesh];
     const int64_t NG = A.N + A.G;
     cudaStream_t s = (cudaStream_t)gbGetStream();
-    float* stage = nullptr;
-    if (!ok_(cudaMalloc((void**)&stage, NG * 5 * sizeof(float)), "gbBatchGetState")) return 1;
+    std::lock_guard<std::mutex> lock(b->ws.mu);
+    if (!b->ws.ensure((size_t)NG * 5 * sizeof(float), "gbBatchGetState")) return 1;
+    float* stage = (float*)b->ws.dev;
     const int cur = I.cur;
-    launch_gather_scalar(NG, I.rho[cur], A.d_cell_new, stage, s);
-    launch_gather_vector(NG, I.rhou[cur], A.d_cell_new, stage + NG, s);
-    launch_gather_scalar(NG, I.rhoe[cur], A.d_cell_new, stage + 4 * NG, s);
+    launch_gather_state(NG, I.rho[cur], I.rhou[cur], I.rhoe[cur], A.d_cell_new, stage, s);
     bool ok = ok_(cudaMemcpyAsync(rho, stage, NG * 4, cudaMemcpyDeviceToHost, s), "gbBatchGetState") &&
               ok_(cudaMemcpyAsync(rhou, stage + NG, NG * 12, cudaMemcpyDeviceToHost, s), "gbBatchGetState") &&
-              ok_(cudaMemcpyAsync(rhoe, stage + 4 * NG, NG * 4, cudaMemcpyDeviceToHost, s), "gbBatchGetState") &&
-              ok_(cudaStreamSynchronize(s), "gbBatchGetState");
-    cudaFree(stage);
+              ok_(cudaMemcpyAsync(rhoe, stage + 4 * NG, NG * 4, cudaMemcpyDeviceToHost, s), "gbBatchGetState");
+    ok = ok_(cudaStreamSynchronize(s), "gbBatchGetState") && ok;
     return ok ? 0 : 1;
 }
 
@@ -936,6 +961,7 @@ int gbBatchAutotune(gbBatch* b, gb_scalar cfl, int trial_iters, int* tile_out, i
             for (int sched = 0; sched < 2; ++sched)
                 for (int tile : tiles) cands.push_back(Tuning{tile, sched, var});
         auto trial = [&](const Tuning& c, int iters) -> float {
+            b->exec_key.clear();
             b->h_inst = base;
             b->tile = c.tile;
             b->schedule = c.schedule;
@@ -997,15 +1023,26 @@ int64_t gbBatchRun(gbBatch* b, gb_scalar cfl, int64_t max_iter, double tolerance
     if (check_every <= 0) check_every = 100;
     if (!download_inst(b)) return -1;
     double* d_hist = nullptr;
-    if (history && max_iter > 0) {
-        if (!ok_(cudaMalloc((void**)&d_hist, (size_t)b->n_inst * max_iter * sizeof(double)), "gbBatchRun") ||
-            !ok_(cudaMemsetAsync(d_hist, 0, (size_t)b->n_inst * max_iter * sizeof(double), (cudaStream_t)gbGetStream()),
-                 "gbBatchRun"))
+    const size_t n_hist = history && max_iter > 0 ? (size_t)b->n_inst * max_iter : 0;
+    const bool keep_hist = n_hist <= kHistKeep;
+    if (n_hist > 0) {
+        if (keep_hist && b->hist_cap < n_hist) {
+            if (b->d_hist) cudaFree(b->d_hist);
+            b->d_hist = nullptr;
+            b->hist_cap = 0;
+            if (!ok_(cudaMalloc((void**)&b->d_hist, n_hist * sizeof(double)), "gbBatchRun")) return -1;
+            b->hist_cap = n_hist;
+        }
+        d_hist = b->d_hist;
+        if (!keep_hist && !ok_(cudaMalloc((void**)&d_hist, n_hist * sizeof(double)), "gbBatchRun")) return -1;
+        if (!ok_(cudaMemsetAsync(d_hist, 0, n_hist * sizeof(double), (cudaStream_t)gbGetStream()), "gbBatchRun")) {
+            if (!keep_hist) cudaFree(d_hist);
             return -1;
+        }
         for (int i = 0; i < b->n_inst; ++i) b->h_inst[i].hist = d_hist + (size_t)i * max_iter;
     }
     reset_counters(b, max_iter, history != nullptr);
-    if (!upload_inst(b)) { if (d_hist) cudaFree(d_hist); return -1; }
+    if (!upload_inst(b)) { if (d_hist && !keep_hist) cudaFree(d_hist); return -1; }
     const int64_t done = max_iter > 0 ? run_loop(b, cfl, max_iter, tolerance, check_every) : 0;
     if (done > 0) {
         uint32_t g_max = 0;
@@ -1016,13 +1053,14 @@ int64_t gbBatchRun(gbBatch* b, gb_scalar cfl, int64_t max_iter, double tolerance
             count_launch();
         }
     }
-    bool ok = done >= 0 && ok_(cudaGetLastError(), "gbBatchRun") && download_inst(b);
+    bool ok = done >= 0 && ok_(cudaGetLastError(), "gbBatchRun") && download_inst(b) &&
+              ok_(cudaStreamSynchronize((cudaStream_t)gbGetStream()), "gbBatchRun");
     if (ok && history) {
-        ok = ok_(cudaMemcpy(history, d_hist, (size_t)b->n_inst * max_iter * sizeof(double), cudaMemcpyDeviceToHost),
-                 "gbBatchRun");
+        if (n_hist > 0)
+            ok = ok_(cudaMemcpy(history, d_hist, n_hist * sizeof(double), cudaMemcpyDeviceToHost), "gbBatchRun");
     }
     if (d_hist) {
-        cudaFree(d_hist);
+        if (!keep_hist) cudaFree(d_hist);
         for (InstDev& I : b->h_inst) I.hist = nullptr;
         upload_inst(b);
     }

@@ -34,12 +34,17 @@ namespace {
 constexpr int kFluxBlocksPerSM = GB_FLUX_BLOCKS;
 constexpr int kGradBlocksPerSM = GB_GRAD_BLOCKS;
 
-__global__ void k_init(int64_t n, float* rho, float4* rhou, float* rhoe, float r, float3 ru, float e) {
+__global__ void k_init(int64_t n, float* rho0, float* rho1, float4* rhou0, float4* rhou1, float* rhoe0, float* rhoe1,
+                       float r, float3 ru, float e) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    rho[i] = r;
-    rhou[i] = make_float4(ru.x, ru.y, ru.z, 0.f);
-    rhoe[i] = e;
+    const float4 u = make_float4(ru.x, ru.y, ru.z, 0.f);
+    rho0[i] = r;
+    rho1[i] = r;
+    rhou0[i] = u;
+    rhou1[i] = u;
+    rhoe0[i] = e;
+    rhoe1[i] = e;
 }
 
 struct GhostBuf {
@@ -267,6 +272,30 @@ __global__ void k_scatter_vector(int64_t n, const float* __restrict__ src, const
     if (i < n) dst[idx[i]] = make_float4(src[3 * i], src[3 * i + 1], src[3 * i + 2], 0.f);
 }
 
+__global__ void k_gather_state(int64_t n, const float* __restrict__ rho, const float4* __restrict__ rhou,
+                               const float* __restrict__ rhoe, const uint32_t* __restrict__ idx, float* stage) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t k = idx[i];
+    const float4 u = rhou[k];
+    stage[i] = rho[k];
+    float* s3 = stage + n + 3 * i;
+    s3[0] = u.x; s3[1] = u.y; s3[2] = u.z;
+    stage[4 * n + i] = rhoe[k];
+}
+__global__ void k_scatter_state(int64_t n, const float* __restrict__ stage, const uint32_t* __restrict__ idx,
+                                float* rho0, float* rho1, float4* rhou0, float4* rhou1, float* rhoe0, float* rhoe1) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t k = idx[i];
+    const float* s3 = stage + n + 3 * i;
+    const float r = stage[i], e = stage[4 * n + i];
+    const float4 u = make_float4(s3[0], s3[1], s3[2], 0.f);
+    rho0[k] = r; rho1[k] = r;
+    rhou0[k] = u; rhou1[k] = u;
+    rhoe0[k] = e; rhoe1[k] = e;
+}
+
 inline unsigned grid(int64_t n) { return (unsigned)((n + kBlock - 1) / kBlock); }
 
 }  // namespace
@@ -278,9 +307,10 @@ int reduce_blocks(int64_t n) {
     return (int)b;
 }
 
-void launch_init(int64_t n, float* rho, float4* rhou, float* rhoe, float r, float3 ru, float e, cudaStream_t s) {
+void launch_init(int64_t n, float* const rho[2], float4* const rhou[2], float* const rhoe[2], float r, float3 ru,
+                 float e, cudaStream_t s) {
     if (n == 0) return;
-    k_init<<<grid(n), kBlock, 0, s>>>(n, rho, rhou, rhoe, r, ru, e);
+    k_init<<<grid(n), kBlock, 0, s>>>(n, rho[0], rho[1], rhou[0], rhou[1], rhoe[0], rhoe[1], r, ru, e);
     count_launch();
 }
 
@@ -390,6 +420,19 @@ void launch_scatter_scalar(int64_t n, const float* src, const uint32_t* idx, flo
 void launch_scatter_vector(int64_t n, const float* src3, const uint32_t* idx, float4* dst, cudaStream_t s) {
     if (n == 0) return;
     k_scatter_vector<<<grid(n), kBlock, 0, s>>>(n, src3, idx, dst);
+    count_launch();
+}
+
+void launch_gather_state(int64_t n, const float* rho, const float4* rhou, const float* rhoe, const uint32_t* idx,
+                         float* stage, cudaStream_t s) {
+    if (n == 0) return;
+    k_gather_state<<<grid(n), kBlock, 0, s>>>(n, rho, rhou, rhoe, idx, stage);
+    count_launch();
+}
+void launch_scatter_state(int64_t n, const float* stage, const uint32_t* idx, float* const rho[2],
+                          float4* const rhou[2], float* const rhoe[2], cudaStream_t s) {
+    if (n == 0) return;
+    k_scatter_state<<<grid(n), kBlock, 0, s>>>(n, stage, idx, rho[0], rho[1], rhou[0], rhou[1], rhoe[0], rhoe[1]);
     count_launch();
 }
 

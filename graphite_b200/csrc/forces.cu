@@ -77,15 +77,15 @@ bool wall_force(const MeshAccess& A, unsigned region, const float* rho, const fl
         force[0] = force[1] = force[2] = 0.0;
         return true;
     }
-    double* d = nullptr;
-    if (!ok_(cudaMalloc((void**)&d, (3 * (size_t)blocks + 3) * sizeof(double)), what)) return false;
+    std::lock_guard<std::mutex> lock(A.ws->mu);
+    if (!A.ws->ensure(3 * (size_t)blocks * sizeof(double), what)) return false;
+    double* d = (double*)A.ws->dev;
     k_force_partials<<<blocks, kForceBlock, 0, s>>>(A.dev->ghost, g0, g1, A.dev->cell_geo, A.dev->face_geo, rho, rhou, rhoe, d);
-    k_force_final<<<1, 32, 0, s>>>(d, blocks, d + 3 * blocks);
+    k_force_final<<<1, 32, 0, s>>>(d, blocks, A.ws->host);
     count_launch(2);
-    const bool ok = ok_(cudaGetLastError(), what) &&
-                    ok_(cudaMemcpyAsync(force, d + 3 * blocks, 3 * sizeof(double), cudaMemcpyDeviceToHost, s), what) &&
-                    ok_(cudaStreamSynchronize(s), what);
-    cudaFree(d);
+    const bool ok = ok_(cudaGetLastError(), what) && ok_(cudaStreamSynchronize(s), what);
+    if (ok)
+        for (int k = 0; k < 3; ++k) force[k] = A.ws->host[k];
     return ok;
 }
 

@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 
 #include "graphite_b200.h"
 
@@ -116,7 +117,9 @@ void launch_layout(const DevMesh& m, const uint32_t* cell_old, const uint32_t* f
                    const double* minv, cudaStream_t s);
 
 // ---- Euler path, euler.cu ----
-void launch_init(int64_t n, float* rho, float4* rhou, float* rhoe, float r, float3 ru, float e, cudaStream_t s);
+// the uniform state (r, ru, e) in both value buffers
+void launch_init(int64_t n, float* const rho[2], float4* const rhou[2], float* const rhoe[2], float r, float3 ru,
+                 float e, cudaStream_t s);
 void launch_bc_slip(const DevMesh& m, uint32_t g0, uint32_t g1, float* rho[2], float4* rhou[2], float* rhoe[2],
                     int cur, cudaStream_t s);
 void launch_bc_farfield(const DevMesh& m, uint32_t g0, uint32_t g1, float* rho[2], float4* rhou[2],
@@ -199,11 +202,32 @@ void launch_gather_scalar(int64_t n, const float* src, const uint32_t* idx, floa
 void launch_gather_vector(int64_t n, const float4* src, const uint32_t* idx, float* dst3, cudaStream_t s);
 void launch_scatter_scalar(int64_t n, const float* src, const uint32_t* idx, float* dst, cudaStream_t s);
 void launch_scatter_vector(int64_t n, const float* src3, const uint32_t* idx, float4* dst, cudaStream_t s);
+// a whole state between device order and stage = rho[n], rhou[3n], rhoe[n] in reference order; scatter writes both
+// value buffers
+void launch_gather_state(int64_t n, const float* rho, const float4* rhou, const float* rhoe, const uint32_t* idx,
+                         float* stage, cudaStream_t s);
+void launch_scatter_state(int64_t n, const float* stage, const uint32_t* idx, float* const rho[2],
+                          float4* const rhou[2], float* const rhoe[2], cudaStream_t s);
 
 void count_launch(int n = 1);
 
 struct Topology;
 struct Numbering;
+
+// Device scratch and a pinned result that a mesh, batch or warm start keeps for
+// calls that end with their stream synchronised: a call holds the lock from its
+// first use of them until then, so callers on several threads and streams take
+// turns.  Freed with its owner.
+struct Workspace {
+    std::mutex mu;
+    void* dev = nullptr;
+    size_t dev_bytes = 0;
+    double* host = nullptr;                // pinned, kHostWords doubles, written by kernels directly
+    static constexpr int kHostWords = 4;
+    // at least `bytes` of device scratch and the pinned words; false with the error set
+    bool ensure(size_t bytes, const char* what);
+    ~Workspace();
+};
 
 // Device view of a loaded mesh, for other translation units of the library.
 struct MeshAccess {
@@ -214,6 +238,7 @@ struct MeshAccess {
     int64_t N, G;
     const Topology* topo;                  // host topology (reference numbering)
     const Numbering* num;                  // reference <-> device numbering
+    Workspace* ws;
 };
 bool mesh_access(::cuMesh* mesh, MeshAccess* out);
 bool reference_momentum();

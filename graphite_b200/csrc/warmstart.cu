@@ -19,7 +19,7 @@
 // into registers.  Each CTA writes its gradient once per step into its own
 // slot, and the Adam kernel sums the slots in a fixed order, so training is
 // deterministic.  One training step = train kernel + Adam kernel + step-end
-// kernel, replayed from a CUDA graph.
+// kernel.
 //
 // Inputs are scaled with a fixed squashing map u / sqrt(1 + u^2) of the
 // offset from the wall's centre in units of the wall's extent; outputs are
@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <array>
 #include <cmath>
+#include <mutex>
 #include <random>
 #include <vector>
 
@@ -115,7 +116,8 @@ struct TrainCtl {
 struct Samples {
     // dataset: tile -> (field, 128 consecutive cells)
     const float4* geo;        // [N] (x', y', z', d')
-    const float4* par;        // [F] (Mach, sin AoA, cos AoA, 1)
+    const float4* par;        // [F] (Mach, sin AoA, cos AoA, 1); null: par0 for every field
+    float4 par0;
     const float* target;      // [F][N][5] q - q_freestream
     int64_t n_cells;
     int64_t tiles_per_field;
@@ -311,7 +313,7 @@ __device__ __forceinline__ bool load_sample(const Samples& s, int64_t tile, int 
     }
     if (cell >= s.n_cells) return false;
     const float4 g = s.geo[cell];
-    const float4 p = s.par[field];
+    const float4 p = s.par ? s.par[field] : s.par0;
     f[0] = g.x; f[1] = g.y; f[2] = g.z; f[3] = g.w;
     f[4] = p.x; f[5] = p.y; f[6] = p.z; f[7] = p.w;
     if (s.target) {
@@ -721,6 +723,11 @@ struct gbWarmStartImpl {
     float* d_v = nullptr;
     uint16_t* d_img = nullptr;
     gb::TrainCtl* d_ctl = nullptr;
+    gb::TrainCtl* h_ctl = nullptr;     // pinned
+    std::mutex mu;                     // held by the calls that use the control word and the slots below
+    float* d_partials = nullptr;       // training: per-CTA gradient slots and losses, kept between trainings
+    double* d_lossp = nullptr;
+    int n_slots = 0;
     long long wait_cycles = 0;         // 0: the kernels' default bound
     float4* d_par = nullptr;
     int n_par_alloc = 0;
@@ -773,19 +780,22 @@ void freestream(gb_vector mach, float p, float T, float* q, float4* par) {
     if (par) *par = make_float4(M, sa, ca, 1.0f);
 }
 
-bool check_ctl(WS* w, const char* what) {
-    TrainCtl h{};
-    if (!ok_(cudaMemcpy(&h, w->d_ctl, sizeof(h), cudaMemcpyDeviceToHost), what)) return false;
-    if (h.error) {
-        set_error(std::string(what) + ": a tensor-core wait gave up (stage " + std::to_string(h.error) + ")");
+// Ends the work queued on s and reads its error word back.
+bool check_ctl(WS* w, cudaStream_t s, const char* what) {
+    if (!ok_(cudaMemcpyAsync(w->h_ctl, w->d_ctl, sizeof(TrainCtl), cudaMemcpyDeviceToHost, s), what) ||
+        !ok_(cudaStreamSynchronize(s), what))
+        return false;
+    if (w->h_ctl->error) {
+        set_error(std::string(what) + ": a tensor-core wait gave up (stage " + std::to_string(w->h_ctl->error) + ")");
         return false;
     }
     return true;
 }
 
 bool reset_ctl(WS* w, cudaStream_t s) {
-    const TrainCtl h{0ull, 0.9, 0.999, 0, w->wait_cycles};
-    return ok_(cudaMemcpyAsync(w->d_ctl, &h, sizeof(h), cudaMemcpyHostToDevice, s), "warm start control");
+    // through the pinned copy: every user of it has ended its stream (check_ctl)
+    *w->h_ctl = TrainCtl{0ull, 0.9, 0.999, 0, w->wait_cycles};
+    return ok_(cudaMemcpyAsync(w->d_ctl, w->h_ctl, sizeof(TrainCtl), cudaMemcpyHostToDevice, s), "warm start control");
 }
 
 bool upload_weights(WS* w, const float* host) {
@@ -846,6 +856,7 @@ gbWarmStart* gbWarmStartCreate(cuMesh* mesh, unsigned wall_region, uint64_t seed
               ok_(cudaMalloc((void**)&w->d_img, kImgBytes), "gbWarmStartCreate") &&
               ok_(cudaMemset(w->d_img, 0, kImgBytes), "gbWarmStartCreate") &&
               ok_(cudaMalloc((void**)&w->d_ctl, sizeof(TrainCtl)), "gbWarmStartCreate") &&
+              ok_(cudaMallocHost((void**)&w->h_ctl, sizeof(TrainCtl)), "gbWarmStartCreate") &&
               ok_(cudaMemset(w->d_ctl, 0, sizeof(TrainCtl)), "gbWarmStartCreate");
     // PyTorch-style uniform init, bound 1/sqrt(fan in); the output layer
     // starts small so that the first prediction is close to free stream
@@ -930,8 +941,9 @@ gbWarmStart* gbWarmStartCreate(cuMesh* mesh, unsigned wall_region, uint64_t seed
 void gbWarmStartFree(gbWarmStart* w) {
     if (!w) return;
     for (void* p : {(void*)w->d_geo, (void*)w->d_target, (void*)w->d_w, (void*)w->d_m, (void*)w->d_v,
-                    (void*)w->d_img, (void*)w->d_ctl, (void*)w->d_par})
+                    (void*)w->d_img, (void*)w->d_ctl, (void*)w->d_par, (void*)w->d_partials, (void*)w->d_lossp})
         if (p) cudaFree(p);
+    if (w->h_ctl) cudaFreeHost(w->h_ctl);
     delete w;
 }
 
@@ -1057,6 +1069,7 @@ int64_t gbWarmStartTrain(gbWarmStart* w, int epochs, int tiles_per_cta, float lr
         return -1;
     }
     if (!set_smem_attrs()) return -1;
+    std::lock_guard<std::mutex> lock(w->mu);
     cudaStream_t s = (cudaStream_t)gbGetStream();
     const int64_t nf = (int64_t)w->par.size();
     const int64_t tpf = (w->N + kTile - 1) / kTile;
@@ -1088,16 +1101,25 @@ int64_t gbWarmStartTrain(gbWarmStart* w, int epochs, int tiles_per_cta, float lr
         if (!ok_(cudaMalloc((void**)&w->d_par, nf * sizeof(float4)), "gbWarmStartTrain")) return -1;
         w->n_par_alloc = (int)nf;
     }
-    float* d_partials = nullptr;
-    double* d_lossp = nullptr;
+    if (w->n_slots < grid) {
+        for (void* p : {(void*)w->d_partials, (void*)w->d_lossp})
+            if (p) cudaFree(p);
+        w->d_partials = nullptr;
+        w->d_lossp = nullptr;
+        w->n_slots = 0;
+        if (!ok_(cudaMalloc((void**)&w->d_partials, (size_t)grid * kParams * sizeof(float)), "gbWarmStartTrain") ||
+            !ok_(cudaMalloc((void**)&w->d_lossp, grid * sizeof(double)), "gbWarmStartTrain"))
+            return -1;
+        w->n_slots = grid;
+    }
+    float* const d_partials = w->d_partials;
+    double* const d_lossp = w->d_lossp;
     double* d_hist = nullptr;
     const int64_t per_step = (int64_t)grid * tiles_per_cta;
     const int64_t total = (int64_t)epochs * n_tiles;
     const int64_t n_steps = (total + per_step - 1) / per_step;
     bool ok = ok_(cudaMemcpyAsync(w->d_par, w->par.data(), nf * sizeof(float4), cudaMemcpyHostToDevice, s),
                   "gbWarmStartTrain") &&
-              ok_(cudaMalloc((void**)&d_partials, (size_t)grid * kParams * sizeof(float)), "gbWarmStartTrain") &&
-              ok_(cudaMalloc((void**)&d_lossp, grid * sizeof(double)), "gbWarmStartTrain") &&
               ok_(cudaMemsetAsync(w->d_m, 0, kParams * sizeof(float), s), "gbWarmStartTrain") &&
               ok_(cudaMemsetAsync(w->d_v, 0, kParams * sizeof(float), s), "gbWarmStartTrain") && reset_ctl(w, s);
     if (ok && loss_history && history_len > 0)
@@ -1127,41 +1149,21 @@ int64_t gbWarmStartTrain(gbWarmStart* w, int epochs, int tiles_per_cta, float lr
                                                            w->d_ctl, lr, 0.9f, 0.999f, 1e-8f);
         k_mlp_step_end<<<1, 32, 0, st>>>(w->d_ctl, d_lossp, grid, d_hist, hist_len, loss_norm, 0.9f, 0.999f);
     };
-    // the steps run as a replayed graph of up to 64 steps
-    const int64_t chunk = std::min<int64_t>(64, n_steps);
-    cudaStream_t cap = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    if (ok) {
-        ok = ok_(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking), "gbWarmStartTrain");
-        cudaGraph_t graph = nullptr;
-        ok = ok && ok_(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal), "gbWarmStartTrain");
-        if (ok) {
-            for (int64_t k = 0; k < chunk; ++k) enqueue_step(cap);
-            ok = ok_(cudaStreamEndCapture(cap, &graph), "gbWarmStartTrain") &&
-                 ok_(cudaGraphInstantiate(&exec, graph, 0), "gbWarmStartTrain");
-        }
-        if (graph) cudaGraphDestroy(graph);
-    }
+    // Launched one by one: a step takes about 100 us on the device and its
+    // three launches 6 us on the host, so a graph of 64 steps only added its
+    // own making (0.7 ms per training).
     int64_t done = 0;
-    while (ok && done + chunk <= n_steps) {
-        ok = ok_(cudaGraphLaunch(exec, s), "gbWarmStartTrain");
-        count_launch(3 * (int)chunk);
-        done += chunk;
-        if (ok && (done / chunk) % 64 == 0) ok = ok_(cudaStreamSynchronize(s), "gbWarmStartTrain") && check_ctl(w, "gbWarmStartTrain");
-    }
     while (ok && done < n_steps) {
         enqueue_step(s);
         count_launch(3);
         ++done;
         ok = ok_(cudaGetLastError(), "gbWarmStartTrain");
+        if (ok && done % 4096 == 0) ok = check_ctl(w, s, "gbWarmStartTrain");
     }
-    ok = ok && ok_(cudaStreamSynchronize(s), "gbWarmStartTrain") && check_ctl(w, "gbWarmStartTrain");
+    ok = ok && check_ctl(w, s, "gbWarmStartTrain");
     if (ok && d_hist)
         ok = ok_(cudaMemcpy(loss_history, d_hist, hist_len * sizeof(double), cudaMemcpyDeviceToHost), "gbWarmStartTrain");
-    if (exec) cudaGraphExecDestroy(exec);
-    if (cap) cudaStreamDestroy(cap);
-    for (void* p : {(void*)d_partials, (void*)d_lossp, (void*)d_hist})
-        if (p) cudaFree(p);
+    if (d_hist) cudaFree(d_hist);
     return ok ? n_steps : -1;
 }
 
@@ -1176,6 +1178,7 @@ int gbWarmStartGradient(gbWarmStart* w, int64_t n, const float* x, const float* 
     clear_error();
     if (!w || n <= 0 || !x || !t || !grad) { set_error("gbWarmStartGradient: bad arguments"); return 1; }
     if (!set_smem_attrs()) return 1;
+    std::lock_guard<std::mutex> lock(w->mu);
     cudaStream_t s = (cudaStream_t)gbGetStream();
     const int64_t n_tiles = (n + kTile - 1) / kTile;
     const int tiles_per_cta = 2;
@@ -1210,7 +1213,7 @@ int gbWarmStartGradient(gbWarmStart* w, int64_t n, const float* x, const float* 
              ok_(cudaMemcpyAsync(grad, d_g, kParams * sizeof(float), cudaMemcpyDeviceToHost, s), "gbWarmStartGradient") &&
              ok_(cudaMemcpyAsync(lp.data(), d_lossp, grid * sizeof(double), cudaMemcpyDeviceToHost, s),
                  "gbWarmStartGradient") &&
-             ok_(cudaStreamSynchronize(s), "gbWarmStartGradient") && check_ctl(w, "gbWarmStartGradient");
+             check_ctl(w, s, "gbWarmStartGradient");
         if (ok && loss) {
             double a = 0.0;
             for (double v : lp) a += v;
@@ -1225,6 +1228,7 @@ int gbWarmStartGradient(gbWarmStart* w, int64_t n, const float* x, const float* 
 int gbWarmStartForward(gbWarmStart* w, int64_t n, const float* x, float* y) {
     clear_error();
     if (!w || n <= 0 || !x || !y) { set_error("gbWarmStartForward: bad arguments"); return 1; }
+    std::lock_guard<std::mutex> lock(w->mu);
     cudaStream_t s = (cudaStream_t)gbGetStream();
     DevSamples d;
     float* d_y = nullptr;
@@ -1240,41 +1244,34 @@ int gbWarmStartForward(gbWarmStart* w, int64_t n, const float* x, float* y) {
         fa.y = d_y;
         ok = forward_launch(w, fa, (n + kTile - 1) / kTile, s) &&
              ok_(cudaMemcpyAsync(y, d_y, n * kOutputs * sizeof(float), cudaMemcpyDeviceToHost, s), "gbWarmStartForward") &&
-             ok_(cudaStreamSynchronize(s), "gbWarmStartForward") && check_ctl(w, "gbWarmStartForward");
+             check_ctl(w, s, "gbWarmStartForward");
     }
     if (d_y) cudaFree(d_y);
     return ok ? 0 : 1;
 }
 
 static int predict(WS* w, float* rho[2], float4* rhou[2], float* rhoe[2], gb_vector mach, float p, float T) {
+    std::lock_guard<std::mutex> lock(w->mu);
     cudaStream_t s = (cudaStream_t)gbGetStream();
     float q[5];
     float4 par;
     freestream(mach, p, T, q, &par);
-    float4* d_par1 = nullptr;
-    bool ok = ok_(cudaMalloc((void**)&d_par1, sizeof(float4)), "gbWarmStartPredict") &&
-              ok_(cudaMemcpyAsync(d_par1, &par, sizeof(float4), cudaMemcpyHostToDevice, s), "gbWarmStartPredict") &&
-              reset_ctl(w, s);
-    if (ok) {
-        ForwardArgs fa{};
-        fa.img = reinterpret_cast<const uint4*>(w->d_img);
-        fa.s.geo = w->d_geo;
-        fa.s.par = d_par1;
-        fa.s.n_cells = w->N;
-        fa.s.tiles_per_field = (w->N + kTile - 1) / kTile;
-        fa.s.n_tiles = fa.s.tiles_per_field;
-        fa.ctl = w->d_ctl;
-        fa.rho0 = rho[0]; fa.rho1 = rho[1];
-        fa.rhou0 = rhou[0]; fa.rhou1 = rhou[1];
-        fa.rhoe0 = rhoe[0]; fa.rhoe1 = rhoe[1];
-        for (int k = 0; k < kOutputs; ++k) {
-            fa.qinf[k] = q[k];
-            fa.scale[k] = w->scale[k];
-        }
-        ok = forward_launch(w, fa, fa.s.n_tiles, s) && ok_(cudaStreamSynchronize(s), "gbWarmStartPredict") &&
-             check_ctl(w, "gbWarmStartPredict");
+    ForwardArgs fa{};
+    fa.img = reinterpret_cast<const uint4*>(w->d_img);
+    fa.s.geo = w->d_geo;
+    fa.s.par0 = par;
+    fa.s.n_cells = w->N;
+    fa.s.tiles_per_field = (w->N + kTile - 1) / kTile;
+    fa.s.n_tiles = fa.s.tiles_per_field;
+    fa.ctl = w->d_ctl;
+    fa.rho0 = rho[0]; fa.rho1 = rho[1];
+    fa.rhou0 = rhou[0]; fa.rhou1 = rhou[1];
+    fa.rhoe0 = rhoe[0]; fa.rhoe1 = rhoe[1];
+    for (int k = 0; k < kOutputs; ++k) {
+        fa.qinf[k] = q[k];
+        fa.scale[k] = w->scale[k];
     }
-    if (d_par1) cudaFree(d_par1);
+    const bool ok = reset_ctl(w, s) && forward_launch(w, fa, fa.s.n_tiles, s) && check_ctl(w, s, "gbWarmStartPredict");
     return ok ? 0 : 1;
 }
 
