@@ -569,8 +569,8 @@ int gbNSIWallForce(cuMesh* mesh, FvmField* velocity, FvmField* pressure, unsigne
  * FvmFieldReduceSum, for callers that cannot allocate device memory -- hosts
  * that hand out all device memory from their own pool, plugins whose device
  * footprint must not grow after setup.  It allocates nothing: its scratch is
- * a static array of 4096 partial sums (32 KiB per GPU, held by every GPU that
- * loads the library until exit), so n is limited to 4096 * 2048 = 8,388,608;
+ * a static array of 4096 partial sums (32.5 KiB per GPU with its counters, held
+ * by every GPU that loads the library until exit), so n is limited to 4096 * 2048 = 8,388,608;
  * larger n is rejected with an error.  values and result must be device (or
  * managed) memory; other pointers are rejected.  The first call on each
  * device looks the array's address up (cudaGetSymbolAddress) and keeps it;

@@ -87,3 +87,22 @@ def test_no_alloc_limits_and_reuse():
     _reduce_no_alloc(lib, small, small.numel(), out, stream)     # and the next call works
     torch.cuda.synchronize()
     assert out.item() == 3000.0
+
+
+@pytest.mark.parametrize("n", [1, 3, 2047, 2048, 2049, 4097, 600 * 2048 + 5, 5_000_017])
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+def test_no_alloc_sum_of_every_alignment(n, offset):
+    """Arrays that start and end off a 16-byte boundary, one block and many;
+    the same bits on every call."""
+    import torch
+
+    lib = capi.load()
+    stream = torch.cuda.current_stream().cuda_stream
+    x = (torch.arange(n + offset, device="cuda", dtype=torch.float32) % 1021 - 300.5)[offset:]
+    x[n // 2] = 1e6
+    out = torch.zeros(2, dtype=torch.float64, device="cuda")
+    for k in range(2):
+        _reduce_no_alloc(lib, x, n, out[k:], stream)
+    got = out.cpu()
+    want = float(x.double().sum())               # halves below 2^53: every order gives the exact sum
+    assert got[0].item() == want and got[1].item() == want
