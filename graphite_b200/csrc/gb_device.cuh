@@ -174,8 +174,6 @@ void launch_flux(const DevMesh& m, EulerState q, FaceRecs r, float* rho_n, float
 void launch_reduce_history(int n_partials, const double* partials, const RunCtl* ctl, double* history,
                            unsigned long long history_cap, cudaStream_t s);
 void launch_reduce_partials(int64_t n, const float* v, double* partials, cudaStream_t s);
-// stage 1 with a caller-chosen number of blocks (one partial per block)
-void launch_reduce_partials_blocks(int64_t n, const float* v, double* partials, int blocks, cudaStream_t s);
 // Sum of the partials into out[0]; with ctl (a replayed loop) also the
 // RunCtl bookkeeping above (history may be null).
 void launch_reduce_final(int n_partials, const double* partials, double* out, cudaStream_t s,
@@ -202,6 +200,10 @@ void launch_gather_scalar(int64_t n, const float* src, const uint32_t* idx, floa
 void launch_gather_vector(int64_t n, const float4* src, const uint32_t* idx, float* dst3, cudaStream_t s);
 void launch_scatter_scalar(int64_t n, const float* src, const uint32_t* idx, float* dst, cudaStream_t s);
 void launch_scatter_vector(int64_t n, const float* src3, const uint32_t* idx, float4* dst, cudaStream_t s);
+// a field's gradients + limiters (cell order of the mesh) in the host mirrors' layout and order: g[n][comps][3] and
+// l[n][comps] for n cells and ghosts, a ghost carrying its interior cell's
+void launch_gather_gradients(const DevMesh& m, int comps, const float4* grad, const uint32_t* cell_new, float* g,
+                             float* l, cudaStream_t s);
 // a whole state between device order and stage = rho[n], rhou[3n], rhoe[n] in reference order; scatter writes both
 // value buffers
 void launch_gather_state(int64_t n, const float* rho, const float4* rhou, const float* rhoe, const uint32_t* idx,
