@@ -154,6 +154,11 @@ struct FieldImpl {
     int n_partials = 0;
     bool partials_valid = false;
     float* staging = nullptr;         // size * comps floats
+    // conditions asked for with gbFieldBcFixed / gbFieldBcZeroGrad and not yet
+    // applied: as with the Euler conditions above, one launch applies them all
+    // before anything reads or writes the field
+    FieldBcTable bcs{};
+    bool bcs_pending = false;
 };
 
 MeshImpl* impl(cuMesh* m) { return m ? static_cast<MeshImpl*>(m->impl) : nullptr; }
@@ -350,8 +355,19 @@ bool check_mesh(cuMesh* m) {
     return true;
 }
 
-// Binds a field's device storage to a mesh's cell order (first use).
-bool bind(cuMesh* mesh, FvmField* f, int comps, const char* what) {
+// Applies the field's pending conditions, if any.
+bool flush_field_bcs(cuMesh* mesh, FvmField* f) {
+    FieldImpl* fi = impl(f);
+    if (!fi->bcs_pending) return true;
+    fi->bcs_pending = false;
+    launch_field_bc(impl(mesh)->dev, fi->comps, fi->bcs, fi->cur, fi->val[0], fi->val[1], t_stream);
+    return launch_ok("field boundary conditions");
+}
+
+// Binds a field's device storage to a mesh's cell order (first use).  Every
+// call that uses a field with a mesh comes through here, so its pending
+// conditions are applied here too (keep_bcs: the call adds to them).
+bool bind(cuMesh* mesh, FvmField* f, int comps, const char* what, bool keep_bcs = false) {
     FieldImpl* fi = impl(f);
     if (!fi) { set_error(std::string(what) + ": null field"); return false; }
     if (fi->comps != comps) {
@@ -369,7 +385,7 @@ bool bind(cuMesh* mesh, FvmField* f, int comps, const char* what) {
         return false;
     }
     fi->bound = mesh;
-    return true;
+    return keep_bcs || flush_field_bcs(mesh, f);
 }
 
 bool ensure_grad(cuMesh* mesh, FvmField* f) {
@@ -465,6 +481,7 @@ bool flush_for(const FvmField* f) {
     FieldImpl* fi = impl(f);
     if (!fi || !fi->bound) return true;
     cuMesh* mesh = const_cast<cuMesh*>(fi->bound);
+    if (!flush_field_bcs(mesh, const_cast<FvmField*>(f))) return false;
     const PendingBcs& pb = impl(mesh)->pending;
     if (pb.any && (pb.f[0] == f || pb.f[1] == f || pb.f[2] == f)) return flush_bcs(mesh);
     return true;
@@ -1555,8 +1572,6 @@ namespace gb {
 void launch_fvm_grad(const DevMesh& m, int comps, const float* s, const float4* v, float4* grad, cudaStream_t st);
 void launch_field_init(int64_t n, int comps, void* val0, void* val1, float4 value, int64_t n_grad, float4* grad,
                        cudaStream_t st);
-void launch_field_bc(const DevMesh& m, uint32_t g0, uint32_t g1, int comps, int zero_grad, int cur, void* val0,
-                     void* val1, float4 value, cudaStream_t st);
 void launch_field_axpy(const DevMesh& m, int comps, float a, const void* x, void* y, cudaStream_t st);
 void launch_fvm_apply(const DevMesh& m, int op, const float* s, const float4* v, const float4* g, const float4* phi,
                       float3 phi_c, float* out, cudaStream_t st);
@@ -1580,15 +1595,39 @@ static int field_bc(cuMesh* mesh, FvmField* u, unsigned int region_id, int zero_
     clear_error();
     if (!check_mesh(mesh)) return 1;
     FieldImpl* fi = impl(u);
-    if (!fi || !bind(mesh, u, fi->comps, what) || !flush_for(u)) return 1;
+    if (!fi || !bind(mesh, u, fi->comps, what, true)) return 1;
     MeshImpl* mi = impl(mesh);
+    const PendingBcs& pb = mi->pending;                  // Euler conditions on the field come first
+    if (pb.any && (pb.f[0] == u || pb.f[1] == u || pb.f[2] == u) && !flush_bcs(mesh)) return 1;
     if (region_id >= mi->topo.regions.size()) {
         set_error(std::string(what) + ": no region " + std::to_string(region_id));
         return 1;
     }
-    launch_field_bc(mi->dev, mi->num.region_start[region_id], mi->num.region_start[region_id + 1], fi->comps, zero_grad,
-                    fi->cur, fi->val[0], fi->val[1], make_float4(value.x, value.y, value.z, 0.f), t_stream);
-    return launch_ok(what) ? 0 : 1;
+    // later conditions on a region replace earlier ones; on meshes of more
+    // regions than the table holds each is applied at once
+    const int n_regions = (int)mi->topo.regions.size();
+    const bool table = n_regions <= kMaxFieldRegions;
+    FieldBcTable& tb = fi->bcs;
+    const int r = table ? (int)region_id : 0;
+    if (!fi->bcs_pending) {
+        tb = FieldBcTable{};
+        tb.n = table ? n_regions : 1;
+        for (int k = 0; k < tb.n; ++k) tb.type[k] = -1;
+        for (int k = 0; table && k <= n_regions; ++k) tb.start[k] = mi->num.region_start[k];
+    }
+    tb.type[r] = zero_grad ? 1 : 0;
+    tb.value[r] = make_float4(value.x, value.y, value.z, 0.f);
+    fi->bcs_pending = true;
+    if (table) return 0;
+    // one region of many: the ghosts before it have no condition, those after it neither
+    tb.n = 3;
+    tb.start[0] = (uint32_t)mi->dev.N;
+    tb.start[1] = mi->num.region_start[region_id];
+    tb.start[2] = mi->num.region_start[region_id + 1];
+    tb.type[1] = tb.type[0];
+    tb.value[1] = tb.value[0];
+    tb.type[0] = tb.type[2] = -1;
+    return flush_field_bcs(mesh, u) ? 0 : 1;
 }
 
 int gbFieldBcFixed(cuMesh* mesh, FvmField* u, gb_vector value, unsigned int region_id) {

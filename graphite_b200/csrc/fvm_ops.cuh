@@ -54,27 +54,32 @@ struct OpFace {
     float3 d0, d1, fc;
 };
 
-// face slot k (entry c0 + t N) of cell c0
+// Face slot k (entry c0 + t N) of cell c0.  D: with the offsets d0, d1; FC:
+// with the face centre.  What an operator does not use is not loaded: the
+// face centre of an interior face is two dependent loads away (entry -> face
+// -> centre) and only GB_FVM_SCAL_GRAD_CORRECT reads it.
+template <bool D = true, bool FC = true>
 __device__ __forceinline__ OpFace op_face(const MeshDev& m, uint32_t c0, uint32_t k) {
     OpFace f;
     f.c0 = c0;
     f.c1 = __ldg(&m.nbc[k]);
-    const uint32_t t = __ldg(&m.twin[k]);
-    const bool ghost = t >= m.S;
+    const bool ghost = f.c1 >= m.N;
     f.g1 = ghost ? c0 : f.c1;
     const float4 gk = __ldg(&m.cf_geo[k]);
     f.n = f3(gk);
     f.ds = gk.w;
-    f.d0 = f3(__ldg(&m.df[k]));
-    f.fc = f3(__ldg(&m.face_geo[2 * __ldg(&m.nb[k]).x + 1]));
-    f.d1 = ghost ? f.fc - f3(__ldg(&m.cell_geo[f.c1])) : f3(__ldg(&m.df[t]));
+    if (FC || (D && ghost)) f.fc = f3(__ldg(&m.face_geo[2 * __ldg(&m.nb[k]).x + 1]));
+    if (D) {
+        f.d0 = f3(__ldg(&m.df[k]));
+        f.d1 = ghost ? f.fc - f3(__ldg(&m.cell_geo[f.c1])) : f3(__ldg(&m.df[__ldg(&m.twin[k])]));
+    }
     return f;
 }
 
-template <class F>
+template <bool D = true, bool FC = true, class F>
 __device__ __forceinline__ void for_each_face(const MeshDev& m, uint32_t c0, F&& fn) {
     const uint32_t nf = __ldg(&m.nfc[c0]);
-    for (uint32_t k = c0; k < c0 + nf * m.N; k += m.N) fn(op_face(m, c0, k));
+    for (uint32_t k = c0; k < c0 + nf * m.N; k += m.N) fn(op_face<D, FC>(m, c0, k));
 }
 
 __device__ __forceinline__ float3 grad_of(const float4* g, uint32_t c) { return f3(__ldg(&g[c])); }

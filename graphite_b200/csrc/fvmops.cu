@@ -107,13 +107,13 @@ __device__ __forceinline__ void term_contrib(const TermDev& t, const fvm::OpFace
 
 // sum of coef x operator over the terms, one pass over each cell's faces,
 // into the interior cells of a scalar (OUT = 1) or vector (OUT = 3) field
-template <int OUT>
+template <int OUT, bool D, bool FC>
 __global__ void k_fvm_terms(MeshDev m, TermList terms, float* __restrict__ out_s, float4* __restrict__ out_v) {
     const uint32_t c0 = blockIdx.x * blockDim.x + threadIdx.x;
     if (c0 >= m.N) return;
     float x1 = 0.f;
     float3 x3 = make_float3(0.f, 0.f, 0.f);
-    fvm::for_each_face(m, c0, [&](const fvm::OpFace& f) {
+    fvm::for_each_face<D, FC>(m, c0, [&](const fvm::OpFace& f) {
         for (int q = 0; q < terms.n; ++q) term_contrib<OUT>(terms.t[q], f, x1, x3);
     });
     if (OUT == 1) out_s[c0] = x1;
@@ -134,19 +134,22 @@ __global__ void k_field_init(int64_t n, float* s0, float* s1, float4* v0, float4
 }
 
 // fvmScalarBcFixed (src/fvmops.cu:308-323) and fvmScalarBcZeroGrad /
-// fvmVectorBcZeroGrad (src/fvmops.cu:326-366) on the ghosts [g0, g1) of one
-// region: the given value, or the interior cell's current value, into both
-// buffers.
-__global__ void k_field_bc(uint32_t g0, uint32_t g1, uint32_t N, const uint2* __restrict__ ghost, int zero_grad,
-                           int cur, float* s0, float* s1, float4* v0, float4* v1, float4 value) {
-    const uint32_t t = g0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= g1) return;
+// fvmVectorBcZeroGrad (src/fvmops.cu:326-366) on all ghosts: those of a region
+// with a condition get the given value, or their interior cell's current one,
+// in both buffers.
+__global__ void k_field_bc(uint32_t N, uint32_t G, const uint2* __restrict__ ghost, FieldBcTable tb, int cur, float* s0,
+                           float* s1, float4* v0, float4* v1) {
+    const uint32_t t = N + blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= N + G) return;
+    int k = 0;
+    while (k < tb.n - 1 && t >= tb.start[k + 1]) ++k;
+    if (tb.type[k] < 0) return;
     if (s0) {
-        const float x = zero_grad ? (cur ? s1 : s0)[ghost[t - N].x] : value.x;
+        const float x = tb.type[k] == 1 ? (cur ? s1 : s0)[ghost[t - N].x] : tb.value[k].x;
         s0[t] = x;
         s1[t] = x;
     } else {
-        const float4 x = zero_grad ? (cur ? v1 : v0)[ghost[t - N].x] : value;
+        const float4 x = tb.type[k] == 1 ? (cur ? v1 : v0)[ghost[t - N].x] : tb.value[k];
         v0[t] = x;
         v1[t] = x;
     }
@@ -212,15 +215,15 @@ void launch_field_init(int64_t n, int comps, void* val0, void* val1, float4 valu
     count_launch();
 }
 
-void launch_field_bc(const DevMesh& m, uint32_t g0, uint32_t g1, int comps, int zero_grad, int cur, void* val0,
-                     void* val1, float4 value, cudaStream_t st) {
-    if (g1 <= g0) return;
+void launch_field_bc(const DevMesh& m, int comps, const FieldBcTable& tb, int cur, void* val0, void* val1,
+                     cudaStream_t st) {
+    if (m.G == 0) return;
     if (comps == 1)
-        k_field_bc<<<grid_n(g1 - g0), kBlock, 0, st>>>(g0, g1, (uint32_t)m.N, m.ghost, zero_grad, cur, (float*)val0,
-                                                       (float*)val1, nullptr, nullptr, value);
+        k_field_bc<<<grid_n(m.G), kBlock, 0, st>>>((uint32_t)m.N, (uint32_t)m.G, m.ghost, tb, cur, (float*)val0,
+                                                   (float*)val1, nullptr, nullptr);
     else
-        k_field_bc<<<grid_n(g1 - g0), kBlock, 0, st>>>(g0, g1, (uint32_t)m.N, m.ghost, zero_grad, cur, nullptr, nullptr,
-                                                       (float4*)val0, (float4*)val1, value);
+        k_field_bc<<<grid_n(m.G), kBlock, 0, st>>>((uint32_t)m.N, (uint32_t)m.G, m.ghost, tb, cur, nullptr, nullptr,
+                                                   (float4*)val0, (float4*)val1);
     count_launch();
 }
 
@@ -240,8 +243,19 @@ void launch_fvm_terms(const DevMesh& m, int out_comps, int n_terms, const FvmTer
     tl.n = n_terms;
     for (int q = 0; q < n_terms; ++q)
         tl.t[q] = TermDev{terms[q].op, terms[q].coef, terms[q].s, terms[q].v, terms[q].g, terms[q].phi, terms[q].phi_c};
-    if (out_comps == 1) k_fvm_terms<1><<<grid_n(m.N), kBlock, 0, st>>>(mesh_dev(m), tl, out_s, nullptr);
-    else k_fvm_terms<3><<<grid_n(m.N), kBlock, 0, st>>>(mesh_dev(m), tl, nullptr, out_v);
+    // which parts of a face the operators read: its offsets (face interpolation and second-order convection), its centre
+    bool d = false, fc = false;
+    for (int q = 0; q < n_terms; ++q) {
+        d = d || terms[q].op == 1 || terms[q].op == 2 || terms[q].op == 8;
+        fc = fc || terms[q].op == 2;
+    }
+    const MeshDev md = mesh_dev(m);
+    const unsigned gn = grid_n(m.N);
+    if (out_comps == 1 && !d) k_fvm_terms<1, false, false><<<gn, kBlock, 0, st>>>(md, tl, out_s, nullptr);
+    else if (out_comps == 1) k_fvm_terms<1, true, false><<<gn, kBlock, 0, st>>>(md, tl, out_s, nullptr);
+    else if (!d) k_fvm_terms<3, false, false><<<gn, kBlock, 0, st>>>(md, tl, nullptr, out_v);
+    else if (!fc) k_fvm_terms<3, true, false><<<gn, kBlock, 0, st>>>(md, tl, nullptr, out_v);
+    else k_fvm_terms<3, true, true><<<gn, kBlock, 0, st>>>(md, tl, nullptr, out_v);
     count_launch();
 }
 

@@ -195,6 +195,19 @@ struct FvmTermDev {
 void launch_fvm_terms(const DevMesh& m, int out_comps, int n_terms, const FvmTermDev* terms, float* out_s,
                       float4* out_v, cudaStream_t st);
 
+// Conditions of one field by ghost region (gbFieldBcFixed, gbFieldBcZeroGrad):
+// ghosts [start[r], start[r+1]) get type[r]: -1 none, 0 value[r], 1 their
+// interior cell's value.
+constexpr int kMaxFieldRegions = 16;
+struct FieldBcTable {
+    int n;
+    uint32_t start[kMaxFieldRegions + 1];
+    int type[kMaxFieldRegions];
+    float4 value[kMaxFieldRegions];
+};
+void launch_field_bc(const DevMesh& m, int comps, const FieldBcTable& tb, int cur, void* val0, void* val1,
+                     cudaStream_t st);
+
 // permute helpers for host transfers (new <-> reference order)
 void launch_gather_scalar(int64_t n, const float* src, const uint32_t* idx, float* dst, cudaStream_t s);
 void launch_gather_vector(int64_t n, const float4* src, const uint32_t* idx, float* dst3, cudaStream_t s);
