@@ -10,6 +10,7 @@
 
 #include "euler_loop.cuh"
 #include "gb_device.cuh"
+#include "nsi_loop.cuh"
 #include "gb_internal.h"
 
 namespace gb {
@@ -117,6 +118,7 @@ struct LoopPlan {
     RunCtl* h_ctl = nullptr;
     int64_t cap = 0;
     unsigned int tag = 0;             // first tag no launch has used
+    size_t n_recs = 0;
     void release() {
         for (void* p : {(void*)ghost_off, (void*)recs, (void*)hist, (void*)ctl})
             if (p) cudaFree(p);
@@ -132,7 +134,7 @@ struct MeshImpl {
     uint32_t* d_cell_new = nullptr;   // old -> new, N+G
     PendingBcs pending;
     RunGraphs euler_run, nsi_run;
-    LoopPlan loop;
+    LoopPlan loop, nsi_loop;
     Workspace ws;
     cudaStream_t capture = nullptr;   // stream the loops are captured on
     double* h_result = nullptr;       // pinned: FvmFieldReduceSum's value on the host
@@ -190,6 +192,7 @@ void free_mesh(cuMesh* m) {
         mi->euler_run.release();
         mi->nsi_run.release();
         mi->loop.release();
+        mi->nsi_loop.release();
         if (mi->capture) cudaStreamDestroy(mi->capture);
         if (mi->h_result) cudaFreeHost(mi->h_result);
         delete mi;
@@ -699,25 +702,17 @@ int sm_count() {
     return n;
 }
 
-// Threads per block of the persistent loop on this mesh (a cell each); 0 when
-// its cells do not all fit on the GPU at once.
+// Threads per block of a persistent loop on this mesh (a cell each).
 int loop_threads(const DevMesh& d) {
     const int64_t blocks = kLoopBlocksPerSM * sm_count() - 1;   // one more sums the residual
     const int64_t chunks = (d.N + 31) / 32;
-    const int threads = (int)std::max<int64_t>(64, (chunks + blocks - 1) / blocks * 32);
-    if (threads > kLoopMax || loop_smem(std::max(d.max_faces, 4), threads) > kLoopSmem) return 0;
-    return threads;
+    return (int)std::max<int64_t>(64, (chunks + blocks - 1) / blocks * 32);
 }
 
-size_t loop_recs(const DevMesh& d) {   // records of a plan: states, face states, warp sums, verdict
-    return 2 * 2 * (size_t)d.N + 2 * (size_t)d.S + 2 * (((size_t)d.N + 31) / 32) + 1;
-}
-
-// False when there is no memory for it (nothing is left in the error state: the
-// graphs run instead).
-bool ensure_loop_plan(MeshImpl* mi, int threads, int64_t need) {
-    LoopPlan& lp = mi->loop;
-    const char* what = "gbEulerRun";
+// The plan of a loop with n_recs records (the warp sums and the verdict among
+// them) and a history of `need` iterations.  False when there is no memory for
+// it (nothing is left in the error state: the graphs run instead).
+bool ensure_loop_plan(MeshImpl* mi, LoopPlan& lp, int threads, size_t n_recs, int64_t need, const char* what) {
     const DevMesh& d = mi->dev;
     struct Quiet {
         bool ok = false;
@@ -729,8 +724,9 @@ bool ensure_loop_plan(MeshImpl* mi, int threads, int64_t need) {
     } quiet;
     if (!lp.threads) {
         lp.n_blocks = (int)(((d.N + 31) / 32 + threads / 32 - 1) / (threads / 32));
+        lp.n_recs = n_recs;
         // one set of records for all fields run on the mesh: a launch uses tags no earlier one did
-        if (!dalloc(lp.ghost_off, (size_t)d.G, what) || !dalloc(lp.recs, loop_recs(d), what) ||
+        if (!dalloc(lp.ghost_off, (size_t)d.G, what) || !dalloc(lp.recs, n_recs, what) ||
             !dalloc(lp.ctl, 1, what) || !cuda_ok(cudaMallocHost((void**)&lp.h_ctl, sizeof(RunCtl)), what)) {
             lp.release();
             return false;
@@ -753,10 +749,30 @@ bool ensure_loop_plan(MeshImpl* mi, int threads, int64_t need) {
     return true;
 }
 
+// The arguments that every loop has.  The last records of the plan are the
+// warp sums of the residual and of its density part and the verdict.
+void loop_args(const MeshImpl* mi, const LoopPlan& lp, LoopArgs& a, double tolerance, bool density, double* partials) {
+    const size_t warps = ((size_t)mi->dev.N + 31) / 32;
+    a.N = (uint32_t)mi->dev.N;
+    a.tol = tolerance;
+    a.ctl = lp.ctl;
+    a.hist = lp.hist;
+    a.hist_rho = density ? lp.hist + lp.cap : nullptr;
+    a.hist_cap = (unsigned long long)lp.cap;
+    a.out = mi->dev.red + mi->dev.n_red_max;
+    a.partials = partials;
+    a.n_groups = (int)((mi->dev.N + kBlock - 1) / kBlock);
+    a.n_blocks = lp.n_blocks;
+    a.wsum = lp.recs + lp.n_recs - 1 - 2 * warps;
+    a.wsum_rho = a.wsum + warps;
+    a.verdict = reinterpret_cast<unsigned long long*>(a.wsum_rho + warps);
+}
+size_t loop_tail_recs(const DevMesh& d) { return 2 * (((size_t)d.N + 31) / 32) + 1; }
+
 // Up to n_iter iterations, check_every to a launch; as replay_run_graphs.
-int64_t run_loop(MeshImpl* mi, EulerLoopArgs& a, bool transposed, int& cur, int64_t n_iter, int64_t check_every,
+template <class Launch>
+int64_t run_loop(LoopPlan& lp, LoopArgs& a, Launch&& launch, int& cur, int64_t n_iter, int64_t check_every,
                  std::vector<double>& hist, std::vector<double>* hist2, cudaStream_t s, const char* what) {
-    LoopPlan& lp = mi->loop;
     int64_t done = 0;
     bool ok = cuda_ok(cudaMemsetAsync(lp.ctl, 0, sizeof(RunCtl), s), what);
     while (ok && done < n_iter) {
@@ -765,12 +781,12 @@ int64_t run_loop(MeshImpl* mi, EulerLoopArgs& a, bool transposed, int& cur, int6
         a.cur0 = (int)((cur + done) & 1);
         // no record of an earlier launch carries a tag of this one
         if (lp.tag == 0 || lp.tag > (1u << 31)) {
-            ok = cuda_ok(cudaMemsetAsync(lp.recs, 0, loop_recs(mi->dev) * sizeof(TagRec), s), what);
+            ok = cuda_ok(cudaMemsetAsync(lp.recs, 0, lp.n_recs * sizeof(TagRec), s), what);
             lp.tag = 1;
         }
         a.tag0 = lp.tag;
         lp.tag += (unsigned int)chunk + 1u;
-        ok = ok && cuda_ok(launch_euler_loop(a, mi->dev.max_faces, lp.threads, transposed, s), what) &&
+        ok = ok && cuda_ok(launch(), what) &&
              cuda_ok(cudaMemcpyAsync(hist.data() + done, lp.hist, (size_t)chunk * sizeof(double),
                                      cudaMemcpyDeviceToHost, s), what) &&
              (!hist2 || cuda_ok(cudaMemcpyAsync(hist2->data() + done, lp.hist + lp.cap, (size_t)chunk * sizeof(double),
@@ -1188,14 +1204,16 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
     // against the graphs, us per call of n iterations (B200): 4,608 prisms n = 2
     // 78 / 81, n = 20 248 / 375; 50,000 prisms n = 2 82 / 82, n = 20 292 / 450;
     // 120,000 prisms n = 5 181 / 180, n = 20 474 / 602; 140,736 prisms n = 10
-    // 351 / 336, n = 20 627 / 632, n = 300 27.6 / 30.0 per iteration.
-    const int threads = table_bcs ? loop_threads(mi->dev) : 0;
+    // 351 / 336, n = 20 627 / 632, n = 300 29.1 / 30.0 per iteration.
+    const int threads = loop_threads(mi->dev), faces = std::max(mi->dev.max_faces, 4);
     const int64_t chunk = std::min<int64_t>(check_every, n_iter);
-    const int64_t shortest = threads <= kLoopWide ? 4 : (loop_lean(std::max(mi->dev.max_faces, 4), threads) ? 32 : 8);
-    if (threads > 0 && chunk >= shortest && ensure_loop_plan(mi, threads, chunk)) {
-        const LoopPlan& lp = mi->loop;
-        const size_t N = (size_t)mi->dev.N, warps = (N + 31) / 32;
+    const int64_t shortest = threads <= kLoopWide ? 4 : (loop_lean(faces, threads) ? 32 : 8);
+    const size_t N = (size_t)mi->dev.N, n_recs = 4 * N + 2 * (size_t)mi->dev.S + loop_tail_recs(mi->dev);
+    if (table_bcs && threads <= kLoopMax && loop_smem(faces, threads) <= kLoopSmem && chunk >= shortest &&
+        ensure_loop_plan(mi, mi->loop, threads, n_recs, chunk, "gbEulerRun")) {
+        LoopPlan& lp = mi->loop;
         EulerLoopArgs a{};
+        loop_args(mi, lp, a, tolerance, density, ei->partials);
         a.m = mesh_dev(mi->dev);
         for (int k = 0; k < 2; ++k) {
             a.rho[k] = (float*)impl(rho)->val[k];
@@ -1204,9 +1222,6 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
             a.state[k] = lp.recs + 2 * N * k;
         }
         a.rec = lp.recs + 4 * N;
-        a.wsum = a.rec + 2 * (size_t)mi->dev.S;
-        a.wsum_rho = a.wsum + warps;
-        a.verdict = reinterpret_cast<unsigned long long*>(a.wsum_rho + warps);
         a.rec_rho = (float*)impl(rho)->rec;
         a.rec_rhou = (float4*)impl(rhou)->rec;
         a.err = (float*)ei->val[ei->cur];
@@ -1214,19 +1229,11 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
         gbt.store = 0;
         a.ghosts = gbt;
         a.cfl = cfl;
-        a.tol = tolerance;
-        a.ctl = lp.ctl;
-        a.hist = lp.hist;
-        a.hist_rho = density ? lp.hist + lp.cap : nullptr;
-        a.hist_cap = (unsigned long long)lp.cap;
-        a.out = out;
-        a.partials = ei->partials;
-        a.n_groups = nb;
-        a.n_blocks = lp.n_blocks;
         int cur = impl(rho)->cur;
         std::vector<double> hist((size_t)n_iter, 0.0), hist_rho(density ? (size_t)n_iter : 0, 0.0);
-        const int64_t done = run_loop(mi, a, transposed, cur, n_iter, check_every, hist, density ? &hist_rho : nullptr,
-                                      s, "gbEulerRun");
+        const int64_t done = run_loop(
+            lp, a, [&] { return launch_euler_loop(a, faces, lp.threads, transposed, s); }, cur, n_iter, check_every, hist,
+            density ? &hist_rho : nullptr, s, "gbEulerRun");
         if (done > 0) {
             // what the kernels of an iteration leave behind: the ghost states of the last gradient pass, from the
             // state it read (the buffer before the last update), and its face states
@@ -1492,7 +1499,7 @@ int64_t gbNSIRun(cuMesh* mesh, FvmField* velocity, FvmField* pressure, FvmField*
     const int n_regions = (int)mi->topo.regions.size();
     const bool inline_bcs = n_regions > 0 && n_regions <= kMaxNsiRegions && 4 * mi->dev.G >= mi->dev.N;
     NsiGhostTable gt{};
-    if (inline_bcs) {
+    if (n_regions <= kMaxNsiRegions) {
         gt.n = n_regions;
         for (int r = 0; r <= n_regions; ++r) gt.start[r] = mi->num.region_start[r];
         for (int r = 0; r < n_regions; ++r) gt.type[r] = -1;
@@ -1506,6 +1513,55 @@ int64_t gbNSIRun(cuMesh* mesh, FvmField* velocity, FvmField* pressure, FvmField*
             gt.p[k] = (float*)impl(pressure)->val[k];
             gt.u[k] = (float4*)impl(velocity)->val[k];
         }
+    }
+    // The persistent loop where the mesh fits on the GPU one cell per thread
+    // and a launch pays for loading the cells' geometry (as in euler_run).
+    // Measured per iteration against the graphs, us (B200): 1,152 hexes 7.4 /
+    // 19.9, 28,800 tets 8.3 / 26.6, 60,000 hexes 10.4 / 24.1, 100,000 hexes
+    // 20.1 / 29.1, with the limiter 1,152 hexes 15.1 / 24.0, 110,000 hexes 30.5
+    // / 32.1.
+    const int threads = loop_threads(mi->dev), faces = std::max(mi->dev.max_faces, 4);
+    const int64_t chunk = std::min<int64_t>(check_every, n_iter);
+    const size_t N = (size_t)mi->dev.N, n_recs = (4 + kNsiGradRecs) * N + loop_tail_recs(mi->dev);
+    if (n_regions > 0 && n_regions <= kMaxNsiRegions && threads <= kNsiMax &&
+        nsi_loop_smem(faces, threads) <= kLoopSmem && chunk >= (threads <= kNsiWide ? 4 : 8) &&
+        ensure_loop_plan(mi, mi->nsi_loop, threads, n_recs, chunk, "gbNSIRun")) {
+        LoopPlan& lp = mi->nsi_loop;
+        NsiLoopArgs a{};
+        loop_args(mi, lp, a, tolerance, false, ei->partials);
+        a.m = mesh_dev(mi->dev);
+        a.ghost_off = lp.ghost_off;
+        for (int k = 0; k < 2; ++k) {
+            a.p[k] = (float*)impl(pressure)->val[k];
+            a.u[k] = (float4*)impl(velocity)->val[k];
+            a.state[k] = lp.recs + 2 * N * k;
+        }
+        a.grad = lp.recs + 4 * N;
+        a.err = (float*)ei->val[ei->cur];
+        a.ghosts = gt;
+        a.par = NsiParams{cfl, (float)t_nsi.viscosity, (float)(t_nsi.beta * t_nsi.beta), t_nsi.corrected};
+        a.limited = t_nsi.limited;
+        int cur = impl(pressure)->cur;
+        std::vector<double> hist((size_t)n_iter, 0.0);
+        const int64_t done = run_loop(
+            lp, a, [&] { return launch_nsi_loop(a, faces, lp.threads, s); }, cur, n_iter, check_every, hist, nullptr, s,
+            "gbNSIRun");
+        if (done > 0) {
+            // what the kernels of an iteration leave behind: the ghost states and gradients of the state before the
+            // last update
+            for (int r = 0; r < n_regions; ++r)
+                if (gt.type[r] >= 0)
+                    enqueue_nsi_bc(mesh, velocity, pressure, r, gt.type[r], 1 - cur,
+                                   gb_vector{gt.vinf[r].x, gt.vinf[r].y, gt.vinf[r].z}, gt.pinf[r], s);
+            launch_nsi_grad(mi->dev, (const float*)impl(pressure)->val[1 - cur],
+                            (const float4*)impl(velocity)->val[1 - cur], impl(pressure)->grad, impl(velocity)->grad,
+                            t_nsi.limited, s);
+            if (!launch_ok("gbNSIRun")) return -1;
+        }
+        impl(velocity)->cur = impl(pressure)->cur = cur;
+        ei->partials_valid = true;
+        if (residual_history && done > 0) memcpy(residual_history, hist.data(), (size_t)done * sizeof(double));
+        return done;
     }
     std::vector<uint64_t> key;
     for (const FvmField* f : {velocity, pressure, error}) key_field(key, f);

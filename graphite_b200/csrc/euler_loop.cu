@@ -24,8 +24,10 @@
 // neighbours at once and keeps what it can on chip; beyond that the issue
 // slots, so a thread takes its faces one at a time in few registers.  Measured
 // per iteration against the replayed graph of four kernels (B200): 4,608
-// prisms 10.3 / 17.7 us, 28,800 tets 11.8 / 20.3, 50,000 prisms 12.2 / 21.9,
-// 120,000 prisms 19.5 / 27.5, 140,736 prisms (normals read from L2) 27.6 / 30.0.
+// prisms 10.1 / 17.7 us, 28,800 tets 11.0 / 20.3, 50,000 prisms 12.1 / 21.9,
+// 120,000 prisms 16.8 / 27.5, 140,736 prisms (normals read from L2) 29.1 / 30.0.
+// With a state's two records side by side instead of in planes the 120,000
+// prisms took 19.5.
 // Flags per block instead of tagged data took 12 to 21 us for these: a fence
 // on each side and a block barrier per hand-over, and the slowest warp of
 // every block in everyone's way.
@@ -36,57 +38,19 @@
 namespace gb {
 namespace {
 
-// Polls of a wait before it gives up (a poll takes about half a microsecond).
-constexpr unsigned int kLoopSpinLimit = 1u << 23;
-
-__device__ __forceinline__ TagRec ld_rec(const TagRec* p) {
-    unsigned long long lo, hi;
-    asm volatile(
-        "{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}\n"
-        : "=l"(lo), "=l"(hi)
-        : "l"(p)
-        : "memory");
-    return TagRec{(uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32)};
-}
-__device__ __forceinline__ void st_rec(TagRec* p, uint32_t x, uint32_t y, uint32_t z, uint32_t tag) {
-    const unsigned long long lo = (unsigned long long)y << 32 | x, hi = (unsigned long long)tag << 32 | z;
-    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%0, %1};\n\tst.relaxed.gpu.global.b128 [%2], t;\n\t}\n" ::"l"(lo),
-                 "l"(hi), "l"(p)
-                 : "memory");
-}
-__device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];\n" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_relaxed64(unsigned long long* p, unsigned long long v) {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;\n" ::"l"(p), "l"(v) : "memory");
-}
-
-// Counts the polls of one wait; false once it, or another one, has given up.
-struct Patience {
-    unsigned int n = 0;
-    int* error;
-    __device__ __forceinline__ explicit Patience(int* e) : error(e) {}
-    __device__ __forceinline__ bool more() {
-        if ((++n & 255u) == 0u && (n >= kLoopSpinLimit || *(volatile int*)error)) {
-            atomicExch(error, 1);
-            return false;
-        }
-        return true;
-    }
-};
-
-__device__ __forceinline__ void st_state(TagRec* p, float r, float3 u, float e, unsigned int tag) {
+// A state is two records, `plane` apart: the lanes of a warp read and write
+// whole sectors of each plane (side by side, every 16-byte access would move a
+// 32-byte sector and use half of it).
+__device__ __forceinline__ void st_state(TagRec* p, size_t plane, float r, float3 u, float e, unsigned int tag) {
     st_rec(p, __float_as_uint(r), __float_as_uint(u.x), __float_as_uint(u.y), tag);
-    st_rec(p + 1, __float_as_uint(u.z), __float_as_uint(e), 0u, tag);
+    st_rec(p + plane, __float_as_uint(u.z), __float_as_uint(e), tag, tag);
 }
 // whether both records of a state carry `tag`; their values if so
-__device__ __forceinline__ bool ld_state(const TagRec* p, unsigned int tag, float& r, float4& ue) {
-    const TagRec a = ld_rec(p), b = ld_rec(p + 1);
+__device__ __forceinline__ bool ld_state(const TagRec* p, size_t plane, unsigned int tag, float& r, float4& ue) {
+    const TagRec a = ld_rec(p), b = ld_rec(p + plane);
     r = __uint_as_float(a.x);
     ue = make_float4(__uint_as_float(a.y), __uint_as_float(a.z), __uint_as_float(b.x), __uint_as_float(b.y));
-    return a.tag == tag && b.tag == tag;
+    return fresh<3>(a, tag) && fresh<2>(b, tag);
 }
 
 // One cell's face entries in shared memory, [slot][component][cell of the
@@ -218,7 +182,7 @@ __device__ __forceinline__ bool grad_loop_cell(const EulerLoopArgs& a, int buf, 
 #pragma unroll
             for (int t = 0; t < MAXF; ++t)
                 if (pending & (1u << t))
-                    if (!ld_state(&nbs[2 * (g.nb(t) & kNbMask)], tag, nr[t], nu[t])) left |= 1u << t;
+                    if (!ld_state(&nbs[g.nb(t) & kNbMask], m.N, tag, nr[t], nu[t])) left |= 1u << t;
             pending = left;
             if (pending == 0) break;
             if (!wait.more()) return false;
@@ -234,7 +198,7 @@ __device__ __forceinline__ bool grad_loop_cell(const EulerLoopArgs& a, int buf, 
             float r;
             float4 ue;
             if (j < m.N) {
-                while (!ld_state(&nbs[2 * j], tag, r, ue))
+                while (!ld_state(&nbs[j], m.N, tag, r, ue))
                     if (!wait.more()) return false;
             } else {
                 ue = __ldcg(&a.rhou[buf][j]);
@@ -275,7 +239,7 @@ __device__ __forceinline__ bool grad_loop_cell(const EulerLoopArgs& a, int buf, 
         float3 ru;
         reconstruct<TRANSPOSED>(v[0], u0, v[4], gr, gu, ge, g.df3(t), rr, ru, re);
         const uint32_t j = g.nb(t) & kNbMask;
-        if (j < m.N || !WIDE) st_state(&a.rec[2 * (i + t * m.N)], rr, ru, re, tag);
+        if (j < m.N || !WIDE) st_state(&a.rec[i + t * m.N], m.S, rr, ru, re, tag);
         if (WIDE) {
             g.own(t, 0) = rr; g.own(t, 1) = ru.x; g.own(t, 2) = ru.y; g.own(t, 3) = ru.z; g.own(t, 4) = re;
         }
@@ -333,7 +297,7 @@ __device__ __forceinline__ bool flux_loop_cell(const EulerLoopArgs& a, unsigned 
                                                uint32_t i, int nf, FluxSum& s) {
     const MeshDev& m = a.m;
     Patience wait(&a.ctl->error);
-    auto twin = [&](uint32_t word) { return &a.rec[2 * ((word >> 28) * m.N + (word & kNbMask))]; };
+    auto twin = [&](uint32_t word) { return &a.rec[(word >> 28) * m.N + (word & kNbMask)]; };
     if constexpr (WIDE) {
         float rb[MAXF];
         float4 ub[MAXF];
@@ -363,7 +327,7 @@ __device__ __forceinline__ bool flux_loop_cell(const EulerLoopArgs& a, unsigned 
 #pragma unroll
             for (int t = 0; t < MAXF; ++t)
                 if (pending & (1u << t))
-                    if (!ld_state(twin(g.nb(t)), tag, rb[t], ub[t])) left |= 1u << t;
+                    if (!ld_state(twin(g.nb(t)), m.S, tag, rb[t], ub[t])) left |= 1u << t;
             pending = left;
             if (pending == 0) break;
             if (!wait.more()) return false;
@@ -379,9 +343,9 @@ __device__ __forceinline__ bool flux_loop_cell(const EulerLoopArgs& a, unsigned 
             const uint32_t word = g.nb(t), j = word & kNbMask;
             float ra, rb;
             float4 ua, ub;
-            ld_state(&a.rec[2 * (i + t * m.N)], tag, ra, ua);   // this thread's own stores
+            ld_state(&a.rec[i + t * m.N], m.S, tag, ra, ua);   // this thread's own stores
             if (j < m.N) {
-                while (!ld_state(twin(word), tag, rb, ub))
+                while (!ld_state(twin(word), m.S, tag, rb, ub))
                     if (!wait.more()) return false;
             } else {
                 rb = __ldcg(&a.rec_rho[m.S + (j - m.N)]);
@@ -392,102 +356,6 @@ __device__ __forceinline__ bool flux_loop_cell(const EulerLoopArgs& a, unsigned 
         }
     }
     return true;
-}
-
-__device__ __forceinline__ double warp_sum(double x) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    return x;
-}
-
-// The residual of one iteration from the per-warp sums tagged `tag`, in the
-// order of k_flux's block sums and k_reduce_final: 8 warps to a 256-cell group
-// (into `groups`), the groups strided over 256 (virtual) threads, then the
-// block tree.  Every thread of the block calls it and gets the sum; ok turns
-// false when a wait gave up.
-__device__ double reduce_groups(const TagRec* wsum, uint32_t N, int n_groups, unsigned int tag, double* groups,
-                                int* error, bool& ok) {
-    __shared__ double sv[kBlock];
-    __shared__ double sw[kBlock / 32];
-    const uint32_t n_warps = (N + 31) / 32;
-    Patience wait(error);
-    for (int v = threadIdx.x; v < kBlock; v += blockDim.x) {
-        double s = 0.0;
-        for (int i = v; i < n_groups; i += kBlock) {
-            double w[8];
-            unsigned int pending = 0xffu;
-            while (pending && ok) {
-                unsigned int left = 0;
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    if (!(pending & (1u << k))) continue;
-                    w[k] = 0.0;
-                    if (8u * i + k >= n_warps) continue;
-                    const TagRec r = ld_rec(&wsum[8 * i + k]);
-                    w[k] = __hiloint2double((int)r.y, (int)r.x);
-                    if (r.tag != tag) left |= 1u << k;
-                }
-                pending = left;
-                if (pending) ok = wait.more();
-            }
-            const double g = ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
-            if (groups) groups[i] = g;
-            s += g;
-        }
-        sv[v] = s;
-    }
-    ok = !__syncthreads_or(!ok);
-    const int lane = threadIdx.x & 31;
-    for (int w = threadIdx.x >> 5; w < kBlock / 32; w += blockDim.x >> 5) {
-        const double x = warp_sum(sv[32 * w + lane]);
-        if (lane == 0) sw[w] = x;
-    }
-    __syncthreads();
-    return ((sw[0] + sw[4]) + (sw[2] + sw[6])) + ((sw[1] + sw[5]) + (sw[3] + sw[7]));
-}
-
-// The block after the workers: residual, history and stop test of each
-// iteration (k_reduce_final's).
-__device__ void loop_reducer(const EulerLoopArgs& a) {
-    RunCtl* ctl = a.ctl;
-    const unsigned long long run0 = ctl->it_run;
-    double res0 = ctl->res0;
-    bool ok = true;
-    for (int it = 0; it < a.iters; ++it) {
-        const unsigned int tag = a.tag0 + it;
-        const double bs = reduce_groups(a.wsum, a.m.N, a.n_groups, tag, nullptr, &ctl->error, ok);
-        double rs = 0.0;
-        if (a.hist_rho) {
-            __syncthreads();
-            rs = reduce_groups(a.wsum_rho, a.m.N, a.n_groups, tag, nullptr, &ctl->error, ok);
-        }
-        if (!ok) return;
-        if (run0 + it == 0) res0 = bs;
-        unsigned int halt = 0;
-        if (!(bs == bs) || bs > 1e300) halt = 2;
-        else if (a.tol > 0.0 && res0 > 0.0 && bs / res0 < a.tol) halt = 1;
-        const bool last = halt || it + 1 == a.iters;
-        if (last) {
-            __syncthreads();
-            reduce_groups(a.wsum, a.m.N, a.n_groups, tag, a.partials, &ctl->error, ok);
-        }
-        if (threadIdx.x == 0) {
-            st_relaxed64(a.verdict, (unsigned long long)halt << 32 | tag);
-            if ((unsigned long long)it < a.hist_cap) {
-                a.hist[it] = bs;
-                if (a.hist_rho) a.hist_rho[it] = rs;
-            }
-            if (last) {
-                a.out[0] = bs;
-                ctl->it_chunk = it + 1;
-                ctl->it_run = run0 + it + 1;
-                ctl->res0 = res0;
-                ctl->halt = halt;
-            }
-        }
-        if (last) return;
-        __syncthreads();
-    }
 }
 
 // Thread t of warp w of block b owns cell 32 (w n_blocks + b) + t: the warps
@@ -522,7 +390,7 @@ __global__ void __launch_bounds__(THREADS, kLoopBlocksPerSM) k_euler_loop(const 
         own.r = a.rho[c][i];
         own.u = f3(a.rhou[c][i]);
         own.e = a.rhoe[c][i];
-        st_state(&a.state[c][2 * i], own.r, own.u, own.e, a.tag0);
+        st_state(&a.state[c][i], m.N, own.r, own.u, own.e, a.tag0);
         ghost_states<MAXF, WIDE, LEAN>(a, s_bc, geo, nf, c, own);
     }
     for (int it = 0; it < a.iters; ++it) {
@@ -536,17 +404,7 @@ __global__ void __launch_bounds__(THREADS, kLoopBlocksPerSM) k_euler_loop(const 
             else if (have) ok = flux_loop_cell<MAXF, WIDE, false, LEAN>(a, tag, geo, i, nf, s);
         }
         // the update waits for the verdict on the iteration before it
-        if (ok && it > 0) {
-            Patience wait(&a.ctl->error);
-            for (;;) {
-                const unsigned long long v = ld_relaxed64(a.verdict);
-                if ((unsigned int)v >= tag - 1u) {
-                    ok = (v >> 32) == 0;
-                    break;
-                }
-                if (!wait.more()) { ok = false; break; }
-            }
-        }
+        if (ok && it > 0) ok = await_verdict(a, tag);
         if (!__all_sync(0xffffffffu, ok)) return;
         float e = 0.f, rsq = 0.f;
         if (have) {
@@ -554,20 +412,14 @@ __global__ void __launch_bounds__(THREADS, kLoopBlocksPerSM) k_euler_loop(const 
             own.r = own.r - s.fr * dt;
             own.u = make_float3(own.u.x - s.fu.x * dt, own.u.y - s.fu.y * dt, own.u.z - s.fu.z * dt);
             own.e = own.e - s.fe * dt;
-            st_state(&a.state[nxt][2 * i], own.r, own.u, own.e, tag + 1u);
+            st_state(&a.state[nxt][i], m.N, own.r, own.u, own.e, tag + 1u);
             const float vol = geo.vol();
             // flux_cell's multiply-adds, written out: the density part below must not change them
             e = __fmul_rn(__fmaf_rn(s.fe, s.fe, __fmaf_rn(s.fr, s.fr, ydot(s.fu, s.fu))), vol);
             rsq = __fmul_rn(__fmul_rn(s.fr, s.fr), vol);
         }
-        const double res = warp_sum((double)e);
-        if ((threadIdx.x & 31) == 0)
-            st_rec(&a.wsum[chunk], (uint32_t)__double2loint(res), (uint32_t)__double2hiint(res), 0u, tag);
-        if (a.hist_rho) {
-            const double r = warp_sum((double)rsq);
-            if ((threadIdx.x & 31) == 0)
-                st_rec(&a.wsum_rho[chunk], (uint32_t)__double2loint(r), (uint32_t)__double2hiint(r), 0u, tag);
-        }
+        st_warp_sum(&a.wsum[chunk], (double)e, tag);
+        if (a.hist_rho) st_warp_sum(&a.wsum_rho[chunk], (double)rsq, tag);
         if (have) {
             a.rho[nxt][i] = own.r;
             a.rhou[nxt][i] = make_float4(own.u.x, own.u.y, own.u.z, 0.f);

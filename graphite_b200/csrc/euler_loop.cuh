@@ -1,7 +1,7 @@
 // Arguments and launch of the persistent Euler loop (euler_loop.cu).
 #pragma once
 
-#include "euler_ops.cuh"
+#include "loop.cuh"
 
 namespace gb {
 
@@ -10,21 +10,7 @@ namespace gb {
 constexpr int kLoopWide = 256;
 constexpr int kLoopFull = 416;          // all of a cell's geometry in shared memory up to here
 constexpr int kLoopMax = 512;
-constexpr int kLoopBlocksPerSM = 2;
-constexpr int kLoopSmem = 112 * 1024;   // dynamic shared memory of a block, at most
-
-// 16 bytes that are written and read as one: three words and the tag that
-// says which iteration they belong to.
-struct alignas(16) TagRec {
-    uint32_t x, y, z, tag;
-};
-
-struct LoopVerdict {
-    unsigned int count;     // tag of the last iteration that has been judged
-    unsigned int halt;
-};
-
-struct EulerLoopArgs {
+struct EulerLoopArgs : LoopArgs {
     MeshDev m;
     const float4* ghost_off;              // per ghost: its face centre - its centroid
     float* rho[2];
@@ -35,18 +21,8 @@ struct EulerLoopArgs {
     float* err;
     GhostBcTable ghosts;
     float cfl;
-    int iters, cur0;
-    double tol;
-    RunCtl* ctl;
-    double *hist, *hist_rho;              // hist_rho null: the density part is not summed
-    unsigned long long hist_cap;
-    double *out, *partials;               // the residual, and its sums by 256-cell group
-    int n_groups, n_blocks;
-    unsigned int tag0;                    // tags of this launch: tag0 + iteration
     TagRec* state[2];                     // 2 per cell and buffer: (rho, u, v), (w, E)
     TagRec* rec;                          // 2 per entry: (rho, u, v), (w, E)
-    TagRec *wsum, *wsum_rho;              // per warp: a double
-    unsigned long long* verdict;          // LoopVerdict
 };
 
 // shared memory of a block (bytes); lean: without the face normals and areas

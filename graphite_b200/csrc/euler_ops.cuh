@@ -62,28 +62,26 @@ __device__ __forceinline__ float3 sym_mul(float4 l0, float4 l1, float3 g) {
 // k3 = |d|^3 is shared by the five variables of a face.
 // Where sig = 1 the blend sig + (1 - sig) lim is exactly 1 for the finite
 // lim this function forms, so that case returns before lim is computed.
+// Multiply-adds written out for the same reason as limiter_value's.
 __device__ __forceinline__ float limiter(float u, float3 g, float umin, float umax, float3 d, float k3) {
     const float du = umax - u, dd = umin - u;
-    const float dmm2 = (du - dd) * (du - dd);
+    const float w = __fadd_rn(du, -dd), dmm2 = __fmul_rn(w, w);
     if (dmm2 <= k3) return 1.f;
-    const float delta = dot(g, d);
-    float sig;
+    const float delta = xdot(g, d);
+    float sig = 0.f;
     if (dmm2 <= 2.f * k3) {
-        const float y = dmm2 / k3 - 1.f;
-        sig = 2.f * y * y * y - 3.f * y * y + 1.f;
-    } else {
-        sig = 0.f;
+        const float y = __fadd_rn(dmm2 / k3, -1.f);
+        sig = __fadd_rn(__fmaf_rn(__fmul_rn(__fmul_rn(2.f, y), y), y, -__fmul_rn(__fmul_rn(3.f, y), y)), 1.f);
     }
     float lim = 1.f;
     if (delta > 1e-6f) {
         const float y = du / delta;
-        lim = y < 2.f ? y - 0.25f * y * y : 1.f;
+        lim = y < 2.f ? __fmaf_rn(__fmul_rn(-0.25f, y), y, y) : 1.f;
     } else if (delta < -1e-6f) {
         const float y = dd / delta;
-        lim = y < 2.f ? y - 0.25f * y * y : 1.f;
+        lim = y < 2.f ? __fmaf_rn(__fmul_rn(-0.25f, y), y, y) : 1.f;
     }
-    lim *= 0.8f;
-    return sig + (1.f - sig) * lim;
+    return __fmaf_rn(__fadd_rn(1.f, -sig), __fmul_rn(lim, 0.8f), sig);
 }
 
 // Division and reciprocal in the arithmetic of the Euler path (approximate,

@@ -19,7 +19,7 @@
 // default) the compact correction ((u_j - u_i) - G.d) d / |d|^2 along the
 // centroid offset d, which couples neighbouring cells directly and removes
 // the odd-even decoupling of the plain average.
-#include "euler_ops.cuh"
+#include "nsi_ops.cuh"
 
 namespace gb {
 namespace {
@@ -39,28 +39,6 @@ __global__ void k_nsi_init(int64_t n, float* p, float4* u, float p0, float3 u0) 
 // pressure), 2 no-slip wall (velocity mirrored through zero).  The pressure
 // is extrapolated from the interior except at outflow.  Both value buffers
 // are written.
-// The ghost state of one boundary face from its interior state (pi, ui) and
-// outward normal n.
-__device__ __forceinline__ void nsi_ghost_state(int type, float3 n, float pi, float3 ui, float3 vinf, float pinf,
-                                                float& pg, float3& ug) {
-    // explicitly rounded (xdot): the ghost kernel and the gradient kernel both
-    // form these states and must agree bitwise
-    if (type == 0) {
-        const float s = __fmul_rn(2.f, xdot(n, ui));
-        ug = make_float3(__fmaf_rn(-n.x, s, ui.x), __fmaf_rn(-n.y, s, ui.y), __fmaf_rn(-n.z, s, ui.z));
-        pg = pi;
-    } else if (type == 2) {
-        ug = make_float3(-ui.x, -ui.y, -ui.z);
-        pg = pi;
-    } else if (xdot(vinf, n) < 0.f) {
-        ug = vinf;
-        pg = pi;
-    } else {
-        ug = ui;
-        pg = pinf;
-    }
-}
-
 __global__ void k_nsi_bc(uint32_t g0, uint32_t g1, uint32_t N, const float4* __restrict__ cell_geo,
                          const float4* __restrict__ face_geo, const uint2* __restrict__ ghost, float* pa, float* pb,
                          float4* ua, float4* ub, int cur, int type, float3 vinf, float pinf, const int* halt) {
@@ -157,11 +135,6 @@ __global__ void __launch_bounds__(kBlock, kNsiBlocks)
     for (int a = 0; a < 3; ++a) gu[3 * i + a] = make_float4(gs[a + 1].x, gs[a + 1].y, gs[a + 1].z, lim[a + 1]);
 }
 
-struct NsiParams {
-    float cfl, nu, beta2;
-    int corrected;            // 1: compact correction of the face gradient
-};
-
 __global__ void __launch_bounds__(kBlock, kNsiBlocks)
     k_nsi_flux(MeshDev m, const float* __restrict__ p, const float4* __restrict__ u, const float4* __restrict__ gp,
                const float4* __restrict__ gu, float* __restrict__ p_n, float4* __restrict__ u_n,
@@ -175,8 +148,7 @@ __global__ void __launch_bounds__(kBlock, kNsiBlocks)
         const float3 ui = f3(__ldg(&u[i]));
         const float4 gpi = __ldg(&gp[i]);
         const float4 gui[3] = {__ldg(&gu[3 * i]), __ldg(&gu[3 * i + 1]), __ldg(&gu[3 * i + 2])};
-        float rp = 0.f, sr = 0.f;
-        float3 ru = make_float3(0.f, 0.f, 0.f);
+        NsiSum sum{};
         const uint32_t nf = __ldg(&m.nfc[i]);
         for (uint32_t k = i; k < i + nf * m.N; k += m.N) {
             const uint32_t t = __ldg(&m.twin[k]);
@@ -202,36 +174,11 @@ __global__ void __launch_bounds__(kBlock, kNsiBlocks)
                 gpj = gpi;
                 guj[0] = gui[0]; guj[1] = gui[1]; guj[2] = gui[2];
             }
-            const float pL = pi + dot(f3(gpi), d0) * gpi.w;
-            const float pR = pj + dot(f3(gpj), d1) * gpj.w;
-            const float3 uL = make_float3(ui.x + dot(f3(gui[0]), d0) * gui[0].w, ui.y + dot(f3(gui[1]), d0) * gui[1].w,
-                                          ui.z + dot(f3(gui[2]), d0) * gui[2].w);
-            const float3 uR = make_float3(uj.x + dot(f3(guj[0]), d1) * guj[0].w, uj.y + dot(f3(guj[1]), d1) * guj[1].w,
-                                          uj.z + dot(f3(guj[2]), d1) * guj[2].w);
-            const float unL = dot(uL, n), unR = dot(uR, n);
-            const float lam = fmaxf(fabsf(unL) + sqrtf(unL * unL + P.beta2), fabsf(unR) + sqrtf(unR * unR + P.beta2));
-            const float h = 0.5f * ds;
-            rp += P.beta2 * (unL + unR) * h - lam * h * (pR - pL);
-            ru = ru + (uL * unL + n * pL + uR * unR + n * pR) * h - (uR - uL) * (lam * h);
-            // viscous flux: face gradient of u dotted with n
-            const float3 d = f3(dw);
-            float3 vis;
-            {
-                float g[3];
-                const float du[3] = {uj.x - ui.x, uj.y - ui.y, uj.z - ui.z};
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    const float3 ga = (f3(gui[a]) + f3(guj[a])) * 0.5f;
-                    float gn = dot(ga, n);
-                    if (P.corrected) gn += (du[a] - dot(ga, d)) * dw.w * dot(d, n);
-                    g[a] = gn;
-                }
-                vis = make_float3(g[0], g[1], g[2]);
-            }
-            ru = ru - vis * (P.nu * ds);
-            sr += (lam + 2.f * P.nu * sqrtf(dw.w)) * ds;
+            sum.face(P, pi, ui, gpi, gui, pj, uj, gpj, guj, n, ds, d0, d1, dw);
         }
-        const float dt = P.cfl / sr;
+        const float rp = sum.rp;
+        const float3 ru = sum.ru;
+        const float dt = P.cfl / sum.sr;
         p_n[i] = pi - rp * dt;
         u_n[i] = make_float4(ui.x - ru.x * dt, ui.y - ru.y * dt, ui.z - ru.z * dt, 0.f);
         const float e = (rp * rp + dot(ru, ru)) * vol;

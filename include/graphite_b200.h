@@ -554,7 +554,7 @@ int FvmNSIStepPrepare(cuMesh* mesh, FvmField* velocity, FvmField* pressure);
 /* error[i] = (R_p^2 + |R_u|^2) V, summed by FvmFieldReduceSum */
 int FvmNSIStep(cuMesh* mesh, FvmField* velocity, FvmField* pressure, gb_scalar cfl, const char* time_scheme,
                FvmField* dt, FvmField* error);
-/* The whole loop as replayed graphs (as gbEulerRun).  Boundary conditions:
+/* The whole loop as replayed graphs or a persistent launch (as gbEulerRun).  Boundary conditions:
  * type 0 slip, 1 inlet / outlet (mach = inlet velocity, pressure = outlet
  * pressure), 2 no-slip wall.  The results, ghost values included, are
  * bitwise those of the per-call loop; when the ghosts number at least a
