@@ -12,14 +12,13 @@
 // sample per TMEM lane; the four warps of each lane quarter split each
 // epilogue's columns).  Per tile it runs the
 // forward pass (pre-activations in TMEM, bf16 activations in shared memory),
-// the loss gradient, and the backward pass, recomputing each pre-activation
-// from the stored input of its layer instead of keeping it.  The weight
-// gradients of the two 128x128 layers accumulate in TMEM over all tiles of
-// the launch; the two thin layers' weight gradients are read back per tile
-// into registers.  Each CTA writes its gradient once per step into its own
-// slot, and the Adam kernel sums the slots in a fixed order, so training is
-// deterministic.  One training step = train kernel + Adam kernel + step-end
-// kernel.
+// the loss gradient, and the backward pass, recomputing the pre-activations
+// of layers 1 and 2 from the stored input of their layer instead of keeping
+// them.  The weight gradients of the two 128x128 layers accumulate in TMEM
+// over all tiles of the launch; the two thin layers' weight gradients are read
+// back per tile into registers.  Each CTA writes its gradient once per step
+// into its own slot, and the Adam kernel sums the slots in a fixed order, so
+// training is deterministic.  One training step = train kernel + Adam kernel.
 //
 // Inputs are scaled with a fixed squashing map u / sqrt(1 + u^2) of the
 // offset from the wall's centre in units of the wall's extent; outputs are
@@ -73,12 +72,15 @@ constexpr uint32_t kImgW4 = kImgW3 + kHid * kHid * 2;
 constexpr uint32_t kImgBytes = kImgW4 + kOutPad * kHid * 2;   // 73728
 
 // shared memory map
-constexpr uint32_t kSmX = kImgBytes;                  // [128][16]  bf16
-constexpr uint32_t kSmA1 = kSmX + kTile * kIn * 2;    // [128][128] bf16 (A1, later dZ1)
+constexpr uint32_t kXBytes = kTile * kIn * 2;
+constexpr uint32_t kSmX = kImgBytes;                  // [2][128][16] bf16 (this tile's and the next one's)
+constexpr uint32_t kSmA1 = kSmX + 2 * kXBytes;        // [128][128] bf16
 constexpr uint32_t kSmA2 = kSmA1 + kTile * kHid * 2;  // (A2, later dZ2)
-constexpr uint32_t kSmA3 = kSmA2 + kTile * kHid * 2;  // (A3, later dZ3)
+constexpr uint32_t kSmA3 = kSmA2 + kTile * kHid * 2;
 constexpr uint32_t kSmDY = kSmA3 + kTile * kHid * 2;  // [128][16]
-constexpr uint32_t kSmBytes = kSmDY + kTile * kOutPad * 2;   // 180224
+constexpr uint32_t kSmForward = kSmDY;                // what a forward pass uses
+constexpr uint32_t kSmDZ = kSmDY + kTile * kOutPad * 2;      // [128][128] bf16 (dZ3, later dZ1)
+constexpr uint32_t kSmBytes = kSmDZ + kTile * kHid * 2;      // 217088
 
 // TMEM columns (512 allocated)
 constexpr uint32_t kTmDW2 = 0, kTmDW3 = 128, kTmS1 = 256, kTmS2 = 384;
@@ -106,8 +108,6 @@ __host__ __device__ inline bool padded_param(int p) {
 }
 
 struct TrainCtl {
-    unsigned long long step;
-    double b1t, b2t;          // beta1^(step+1), beta2^(step+1)
     int error;                // stage of a wait that gave up (0 none)
     long long wait_cycles;    // bound of each stage's wait for its MMAs
 };
@@ -133,6 +133,7 @@ struct TrainArgs {
     const uint4* img;         // bf16 weight image
     Samples s;
     TrainCtl* ctl;
+    int64_t step;
     float* partials;          // [grid][kParams]
     double* loss_partials;    // [grid]
     int tiles_per_cta;
@@ -161,14 +162,20 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// 8 values -> bf16 chunk c8 of row r of a buffer with `cols` columns
-__device__ __forceinline__ void put8(uint8_t* buf, int cols, int r, int c8, const float* v) {
+__device__ __forceinline__ uint4 pack8(const float* v) {
     uint4 u;
     u.x = pack_bf16(v[0], v[1]);
     u.y = pack_bf16(v[2], v[3]);
     u.z = pack_bf16(v[4], v[5]);
     u.w = pack_bf16(v[6], v[7]);
+    return u;
+}
+// 8 values -> bf16 chunk c8 of row r of a buffer with `cols` columns
+__device__ __forceinline__ void put8(uint8_t* buf, int cols, int r, int c8, uint4 u) {
     *reinterpret_cast<uint4*>(buf + (r >> 3) * cols * 16 + c8 * 128 + (r & 7) * 16) = u;
+}
+__device__ __forceinline__ void put8(uint8_t* buf, int cols, int r, int c8, const float* v) {
+    put8(buf, cols, r, c8, pack8(v));
 }
 
 __device__ __forceinline__ float tanh_fast(float x) {
@@ -233,30 +240,43 @@ struct Cta {
     uint32_t tm;              // TMEM base
     uint32_t lane;            // this warp's TMEM lane offset (bits 16..)
     int row;                  // TMEM lane = tile row of this thread
-    int group;                // column group; group 0 also does the per-row work
-    uint64_t* bar;
-    uint32_t phase;
+    int group;                // column group
+    uint64_t* bar;            // [0] the stages; [1] MMAs that an epilogue waits for before it stores
+    uint32_t phase;           // bit k: parity of bar[k]
+    bool failed;              // a wait of this thread gave up
+    int* error;
     long long wait;           // SM cycles a stage waits for its MMAs before giving up
 };
 
+__device__ __forceinline__ void await(Cta& c, int k, int where) {
+    if (!umma::bar_wait(c.bar + k, (c.phase >> k) & 1u, c.wait)) {
+        c.failed = true;
+        atomicCAS(c.error, 0, where);
+    }
+    c.phase ^= 1u << k;
+}
+
 // Ends a stage: publishes shared-memory writes to the tensor core, lets thread
-// 0 issue the next MMAs (the callable), and waits for them.  Returns false
-// (on every thread) if the wait gave up.
-template <typename Issue>
-__device__ __forceinline__ bool stage(Cta& c, Issue issue) {
+// 0 issue the next MMAs and commit those the stage waits for (`issue`), runs
+// `shadow` while they work, and waits.  One barrier: a thread whose wait gave
+// up says so at the next stage's.  Returns false (on every thread) then.
+template <typename Issue, typename Shadow>
+__device__ __forceinline__ bool stage(Cta& c, int where, Issue issue, Shadow shadow) {
     umma::fence_smem_async();
     umma::fence_before_sync();
-    __syncthreads();
+    if (__syncthreads_or(c.failed)) return false;
     if (threadIdx.x == 0) {
         umma::fence_after_sync();
         issue();
-        umma::commit(c.bar);
     }
-    const bool ok = umma::bar_wait(c.bar, c.phase, c.wait);
-    c.phase ^= 1u;
-    const bool any_fail = __syncthreads_or(!ok);
+    shadow();
+    await(c, 0, where);
     umma::fence_after_sync();
-    return !any_fail;
+    return true;
+}
+template <typename Issue>
+__device__ __forceinline__ bool stage(Cta& c, int where, Issue issue) {
+    return stage(c, where, issue, [] {});
 }
 
 // S (128 fp32 columns of this thread's row) -> silu -> bf16 row of buf
@@ -273,21 +293,29 @@ __device__ __forceinline__ void epi_silu(const Cta& c, uint32_t s_col, uint8_t* 
     }
 }
 
-// dZ = dA * silu'(Z) with dA in S1, Z in S2 -> bf16 row of buf
-__device__ __forceinline__ void epi_dsilu(const Cta& c, uint8_t* buf) {
+// dZ = dA * silu'(Z) -> bf16 row of buf; `ready` runs before the first store
+template <typename Ready>
+__device__ __forceinline__ void epi_dsilu(const Cta& c, uint32_t da_col, uint32_t z_col, uint8_t* buf, Ready ready) {
     const int r = c.row;
-#pragma unroll 1
-    for (int q = kChunks * c.group; q < kChunks * (c.group + 1); ++q) {
+    uint4 out[kChunks][4];
+#pragma unroll
+    for (int q = 0; q < kChunks; ++q) {
+        const uint32_t col = 32u * (kChunks * c.group + q);
         float da[32], z[32];
-        umma::ld32x2(c.tm + c.lane + kTmS1 + 32u * q, c.tm + c.lane + kTmS2 + 32u * q, da, z);
+        umma::ld32x2(c.tm + c.lane + da_col + col, c.tm + c.lane + z_col + col, da, z);
 #pragma unroll
         for (int k = 0; k < 32; ++k) {
             const float s = sigm(z[k]);
             da[k] *= s * fmaf(z[k], 1.0f - s, 1.0f);
         }
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) put8(buf, kHid, r, 4 * q + cc, da + 8 * cc);
+        for (int cc = 0; cc < 4; ++cc) out[q][cc] = pack8(da + 8 * cc);
     }
+    ready();
+#pragma unroll
+    for (int q = 0; q < kChunks; ++q)
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) put8(buf, kHid, r, 4 * (kChunks * c.group + q) + cc, out[q][cc]);
 }
 
 // sample of this thread in tile `tile`: features f[8], targets tg[5]; false = padding row
@@ -324,25 +352,35 @@ __device__ __forceinline__ bool load_sample(const Samples& s, int64_t tile, int 
     return true;
 }
 
-__device__ __forceinline__ void put_x(uint8_t* sm, int r, bool valid, const float* f) {
+__device__ __forceinline__ void put_x(uint8_t* x, int r, bool valid, const float* f) {
     float v[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) v[k] = valid ? f[k] : 0.0f;
-    put8(sm + kSmX, kIn, r, 0, v);
-    const float zero[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    put8(sm + kSmX, kIn, r, 1, zero);
+    put8(x, kIn, r, 0, v);
+    put8(x, kIn, r, 1, make_uint4(0u, 0u, 0u, 0u));
 }
 
 __device__ __forceinline__ void cta_setup(Cta& c, uint8_t* sm, const uint4* img, uint64_t* bar, uint32_t* slot,
-                                          const TrainCtl* ctl) {
+                                          TrainCtl* ctl) {
     c.sm = sm;
     c.sa = umma::smem_addr(sm);
     c.bar = bar;
     c.phase = 0;
+    c.failed = false;
+    c.error = &ctl->error;
     c.wait = ctl->wait_cycles > 0 ? ctl->wait_cycles : kWaitCycles;
-    for (int k = threadIdx.x; k < (int)(kImgBytes / 16); k += blockDim.x) reinterpret_cast<uint4*>(sm)[k] = img[k];
-    if (threadIdx.x == 0) umma::bar_init(bar, 1);
+    constexpr int kCopies = (int)(kImgBytes / 16) / kThreads;
+    static_assert(kCopies * kThreads * 16 == (int)kImgBytes, "whole rounds of copies");
+    uint4 w[kCopies];
+#pragma unroll
+    for (int k = 0; k < kCopies; ++k) w[k] = img[threadIdx.x + k * kThreads];
+    if (threadIdx.x == 0) {
+        umma::bar_init(bar, 1);
+        umma::bar_init(bar + 1, 1);
+    }
     if (threadIdx.x < 32) umma::tmem_alloc(slot, kTmCols);
+#pragma unroll
+    for (int k = 0; k < kCopies; ++k) reinterpret_cast<uint4*>(sm)[threadIdx.x + k * kThreads] = w[k];
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
@@ -352,15 +390,14 @@ __device__ __forceinline__ void cta_setup(Cta& c, uint8_t* sm, const uint4* img,
     c.group = (int)(threadIdx.x >> 7);
 }
 
-__device__ __forceinline__ void cta_teardown(Cta& c, TrainCtl* ctl, bool ok, int where) {
-    if (!ok) {
-        if (threadIdx.x == 0) atomicCAS(&ctl->error, 0, where);
-        // let any MMA still in flight finish (bounded by the full default,
-        // whatever the stage bound was) before giving TMEM back
-        if (threadIdx.x == 0) {
-            umma::commit(c.bar);
-            umma::bar_wait(c.bar, c.phase, kWaitCycles);
-        }
+__device__ __forceinline__ void cta_teardown(Cta& c, bool ok) {
+    // let any MMA still in flight finish (bounded by the full default,
+    // whatever the stage bound was) before giving TMEM back: first the phase
+    // that a wait may have given up on, then one that covers every MMA
+    if (!ok && threadIdx.x == 0) {
+        umma::bar_wait(c.bar, (c.phase & 1u) ^ 1u, kWaitCycles);
+        umma::commit(c.bar);
+        umma::bar_wait(c.bar, c.phase & 1u, kWaitCycles);
     }
     umma::fence_before_sync();
     __syncthreads();
@@ -370,54 +407,107 @@ __device__ __forceinline__ void cta_teardown(Cta& c, TrainCtl* ctl, bool ok, int
     }
 }
 
-// forward through layers 1-3 (A1..A3 in shared memory) and layer 4 into S2
-__device__ __forceinline__ bool forward(Cta& c) {
-    const uint32_t X = c.sa + kSmX, A1 = c.sa + kSmA1, A2 = c.sa + kSmA2, A3 = c.sa + kSmA3;
-    const uint32_t W1 = c.sa + kImgW1, W2 = c.sa + kImgW2, W3 = c.sa + kImgW3, W4 = c.sa + kImgW4;
-    const uint32_t S1 = c.tm + kTmS1, S2 = c.tm + kTmS2;
-    if (!stage(c, [&] { gemm(S1, X, kIn, false, W1, kIn, false, 128, kHid, kIn, false); })) return false;
-    epi_silu(c, kTmS1, c.sm + kSmA1);
-    if (!stage(c, [&] { gemm(S1, A1, kHid, false, W2, kHid, false, 128, kHid, kHid, false); })) return false;
-    epi_silu(c, kTmS1, c.sm + kSmA2);
-    if (!stage(c, [&] { gemm(S1, A2, kHid, false, W3, kHid, false, 128, kHid, kHid, false); })) return false;
-    epi_silu(c, kTmS1, c.sm + kSmA3);
-    return stage(c, [&] { gemm(S2, A3, kHid, false, W4, kHid, false, 128, kOutPad, kHid, false); });
-}
-
+// One training step's gradient.  Bound by the chain of a tile: seven stages of
+// MMAs (a 128 x 128 x 128 product takes 0.4 us) and epilogues (six with 16,384
+// tanh each, 0.55 us at the SM's rate), one tile in flight because weights and
+// activations fill shared memory and the two accumulators half of TMEM.  So
+// what no epilogue waits for runs beside one: the next tile's samples are read
+// while MMAs work; the weight gradients of layers 2 and 3 run during the
+// epilogues after them; those of the thin layers join the next tile's first
+// stage.  The last pre-activations are still in S1 when their silu' needs
+// them; the others are formed again from the layer's input.  8 tiles on each
+// of 148 SMs: 89.7 us (110 in nine stages with everything waited for).
 __global__ void __launch_bounds__(kThreads, 1) k_mlp_train(const TrainArgs a) {
     extern __shared__ __align__(1024) uint8_t sm[];
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bar[2];
     __shared__ uint32_t slot;
+    const int64_t base = a.step * gridDim.x * a.tiles_per_cta + (int64_t)blockIdx.x * a.tiles_per_cta;
+    const int n_tiles = (int)max((int64_t)0, min((int64_t)a.tiles_per_cta, a.total_slots - base));
     Cta c;
-    cta_setup(c, sm, a.img, &bar, &slot, a.ctl);
+    float f[8], tg[5], tg_next[5];
+    bool valid = false, valid_next = false;
+    // sample of this row in the CTA's tile j
+    auto sample = [&](int j) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) tg_next[k] = 0.0f;
+        const int64_t slot_id = base + j;
+        int64_t tile = slot_id;
+        if (a.permute) {
+            const int64_t epoch = slot_id / a.s.n_tiles;
+            tile = permute_index(slot_id - epoch * a.s.n_tiles, a.s.n_tiles,
+                                 a.seed ^ (0x9E3779B97F4A7C15ull * (epoch + 1)));
+        }
+        valid_next = load_sample(a.s, tile, -1, c.row, f, tg_next);
+    };
+    cta_setup(c, sm, a.img, bar, &slot, a.ctl);
     const int r = c.row;
-    const bool rowwork = c.group == 0;   // the per-row work (sample, loss, thin layers) is done by group 0
-    const uint32_t X = c.sa + kSmX, A1 = c.sa + kSmA1, A2 = c.sa + kSmA2, A3 = c.sa + kSmA3, DY = c.sa + kSmDY;
+    const bool rowwork = c.group == 0;               // samples and loss
+    const bool thinwork = c.group == kGroups - 1;    // weight gradients of the thin layers
+    const uint32_t A1 = c.sa + kSmA1, A2 = c.sa + kSmA2, A3 = c.sa + kSmA3, DY = c.sa + kSmDY, DZ = c.sa + kSmDZ;
     const uint32_t W1 = c.sa + kImgW1, W2 = c.sa + kImgW2, W3 = c.sa + kImgW3, W4 = c.sa + kImgW4;
     const uint32_t S1 = c.tm + kTmS1, S2 = c.tm + kTmS2, DW2 = c.tm + kTmDW2, DW3 = c.tm + kTmDW3;
     float acc1[16], acc4[16];      // this thread's hidden unit: dW1[r][:], dW4[:][r]
 #pragma unroll
     for (int k = 0; k < 16; ++k) acc1[k] = acc4[k] = 0.0f;
     double loss = 0.0;
-    bool first = true, ok = true;
-    int where = 0;
-    const unsigned long long step = a.ctl->step;
-    for (int j = 0; j < a.tiles_per_cta && ok; ++j) {
-        const int64_t slot_id = (int64_t)step * gridDim.x * a.tiles_per_cta + (int64_t)blockIdx.x * a.tiles_per_cta + j;
-        if (slot_id >= a.total_slots) break;
-        int64_t tile = slot_id;
-        if (a.permute) {
-            const int64_t epoch = slot_id / a.s.n_tiles;
-            tile = permute_index(slot_id % a.s.n_tiles, a.s.n_tiles, a.seed ^ (0x9E3779B97F4A7C15ull * (epoch + 1)));
+    // dW1 = dZ1^T X and dW4^T = A3^T dY of the tile before -> S2, and their sums
+    auto thin_mmas = [&](int j) {
+        gemm(S2, DZ, kHid, true, c.sa + kSmX + (j & 1) * kXBytes, kIn, true, 128, kIn, kTile, false);
+        gemm(S2 + kIn, A3, kHid, true, DY, kOutPad, true, 128, kOutPad, kTile, false);
+    };
+    auto thin_sums = [&] {
+        float v[32];
+        umma::ld32(S2 + c.lane, v);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            acc1[k] += v[k];
+            acc4[k] += v[16 + k];
         }
-        float f[8], tg[5] = {0, 0, 0, 0, 0};
-        bool valid = false;
-        if (rowwork) {
-            valid = load_sample(a.s, tile, -1, r, f, tg);
-            put_x(c.sm, r, valid, f);
-        }
-        where = 1;
-        if (!(ok = forward(c))) break;
+    };
+    if (rowwork && n_tiles > 0) {
+        sample(0);
+        put_x(c.sm + kSmX, r, valid_next, f);
+    }
+    bool ok = true;
+    for (int j = 0; j < n_tiles; ++j) {
+        const uint32_t X = c.sa + kSmX + (j & 1) * kXBytes;
+        valid = valid_next;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) tg[k] = tg_next[k];
+        if (!(ok = stage(c, 1, [&] {
+                  gemm(S1, X, kIn, false, W1, kIn, false, 128, kHid, kIn, false);
+                  umma::commit(c.bar);
+                  if (j > 0) thin_mmas(j - 1);
+              })))
+            break;
+        epi_silu(c, kTmS1, c.sm + kSmA1);
+        if (!(ok = stage(
+                  c, 2,
+                  [&] {
+                      gemm(S1, A1, kHid, false, W2, kHid, false, 128, kHid, kHid, false);
+                      umma::commit(c.bar);
+                  },
+                  [&] { if (rowwork && j + 1 < n_tiles) sample(j + 1); })))
+            break;
+        if (thinwork && j > 0) thin_sums();
+        epi_silu(c, kTmS1, c.sm + kSmA2);
+        if (!(ok = stage(
+                  c, 3,
+                  [&] {
+                      gemm(S1, A2, kHid, false, W3, kHid, false, 128, kHid, kHid, false);
+                      umma::commit(c.bar);
+                  },
+                  [&] {
+                      if (rowwork && j + 1 < n_tiles)
+                          put_x(c.sm + kSmX + ((j + 1) & 1) * kXBytes, r, valid_next, f);
+                  })))
+            break;
+        epi_silu(c, kTmS1, c.sm + kSmA3);
+        if (!(ok = stage(c, 4, [&] {
+                  gemm(S2, A3, kHid, false, W4, kHid, false, 128, kOutPad, kHid, false);
+                  umma::commit(c.bar);
+              })))
+            break;
         // loss gradient: dY = dy_scale * (y - t) on valid rows
         if (rowwork) {
             float y[16];
@@ -436,52 +526,41 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_train(const TrainArgs a) {
             put8(c.sm + kSmDY, kOutPad, r, 0, dy);
             put8(c.sm + kSmDY, kOutPad, r, 1, dy + 8);
         }
-        where = 2;
-        // dW4^T (this tile) = A3^T dY -> S2
-        if (!(ok = stage(c, [&] { gemm(S2, A3, kHid, true, DY, kOutPad, true, 128, kOutPad, kTile, false); }))) break;
-        if (rowwork) {
-            float v[16];
-            umma::ld16(S2 + c.lane, v);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) acc4[k] += v[k];
-        }
-        where = 3;
-        // dA3 = dY W4 -> S1; Z3 = A2 W3^T -> S2
-        if (!(ok = stage(c, [&] {
-                  gemm(S1, DY, kOutPad, false, W4, kHid, true, 128, kHid, kOutPad, false);
-                  gemm(S2, A2, kHid, false, W3, kHid, false, 128, kHid, kHid, false);
+        // dA3 = dY W4 -> S2 beside Z3 in S1
+        if (!(ok = stage(c, 5, [&] {
+                  gemm(S2, DY, kOutPad, false, W4, kHid, true, 128, kHid, kOutPad, false);
+                  umma::commit(c.bar);
               })))
             break;
-        epi_dsilu(c, c.sm + kSmA3);            // dZ3 over A3
-        where = 4;
-        // dA2 = dZ3 W3 -> S1; dW3 += dZ3^T A2; Z2 = A1 W2^T -> S2
-        if (!(ok = stage(c, [&] {
-                  gemm(S1, A3, kHid, false, W3, kHid, true, 128, kHid, kHid, false);
-                  gemm(DW3, A3, kHid, true, A2, kHid, true, 128, kHid, kTile, !first);
+        epi_dsilu(c, kTmS2, kTmS1, c.sm + kSmDZ, [] {});         // dZ3
+        // dA2 = dZ3 W3 -> S1; Z2 = A1 W2^T -> S2; dW3 += dZ3^T A2, done before dZ2 goes over A2
+        if (!(ok = stage(c, 6, [&] {
+                  gemm(S1, DZ, kHid, false, W3, kHid, true, 128, kHid, kHid, false);
                   gemm(S2, A1, kHid, false, W2, kHid, false, 128, kHid, kHid, false);
+                  umma::commit(c.bar);
+                  gemm(DW3, DZ, kHid, true, A2, kHid, true, 128, kHid, kTile, j > 0);
+                  umma::commit(c.bar + 1);
               })))
             break;
-        epi_dsilu(c, c.sm + kSmA2);            // dZ2 over A2
-        where = 5;
-        // dA1 = dZ2 W2 -> S1; dW2 += dZ2^T A1; Z1 = X W1^T -> S2
-        if (!(ok = stage(c, [&] {
+        epi_dsilu(c, kTmS1, kTmS2, c.sm + kSmA2, [&] { await(c, 1, 6); });   // dZ2
+        // dA1 = dZ2 W2 -> S1; Z1 = X W1^T -> S2; dW2 += dZ2^T A1, done by the next stage's commit
+        if (!(ok = stage(c, 7, [&] {
                   gemm(S1, A2, kHid, false, W2, kHid, true, 128, kHid, kHid, false);
-                  gemm(DW2, A2, kHid, true, A1, kHid, true, 128, kHid, kTile, !first);
                   gemm(S2, X, kIn, false, W1, kIn, false, 128, kHid, kIn, false);
+                  umma::commit(c.bar);
+                  gemm(DW2, A2, kHid, true, A1, kHid, true, 128, kHid, kTile, j > 0);
               })))
             break;
-        first = false;
-        epi_dsilu(c, c.sm + kSmA1);            // dZ1 over A1
-        where = 6;
-        // dW1 (this tile) = dZ1^T X -> S1
-        if (!(ok = stage(c, [&] { gemm(S1, A1, kHid, true, X, kIn, true, 128, kIn, kTile, false); }))) break;
-        if (rowwork) {
-            float v[16];
-            umma::ld16(S1 + c.lane, v);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) acc1[k] += v[k];
-        }
+        epi_dsilu(c, kTmS1, kTmS2, c.sm + kSmDZ, [] {});         // dZ1 over dZ3
     }
+    if (ok && n_tiles > 0) {
+        ok = stage(c, 8, [&] {
+            thin_mmas(n_tiles - 1);
+            umma::commit(c.bar);
+        });
+        if (ok && thinwork) thin_sums();
+    }
+    ok = !__syncthreads_or(!ok || c.failed);
     if (ok) {
         float* P = a.partials + (size_t)blockIdx.x * kParams;
         // the first half of the groups drains dW2, the second dW3 (row r =
@@ -493,7 +572,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_train(const TrainArgs a) {
 #pragma unroll 1
         for (int q = q0; q < q0 + 8 / kGroups; ++q) {
             float v2[32];
-            if (first) {
+            if (n_tiles == 0) {
 #pragma unroll
                 for (int k = 0; k < 32; ++k) v2[k] = 0.0f;
             } else {
@@ -503,7 +582,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_train(const TrainArgs a) {
 #pragma unroll
             for (int k = 0; k < 8; ++k) p2[k] = make_float4(v2[4 * k], v2[4 * k + 1], v2[4 * k + 2], v2[4 * k + 3]);
         }
-        if (rowwork) {
+        if (thinwork) {
 #pragma unroll
             for (int k = 0; k < 16; ++k) {
                 P[kOffW1 + r * kIn + k] = acc1[k];
@@ -514,46 +593,71 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_train(const TrainArgs a) {
         __shared__ double red[kThreads];
         red[threadIdx.x] = loss;
         __syncthreads();
-        if (r == 0) {
+        if (threadIdx.x == 0) {
             double s = 0.0;
             for (int k = 0; k < kThreads; ++k) s += red[k];
             a.loss_partials[blockIdx.x] = s;
         }
     }
-    cta_teardown(c, a.ctl, ok, where);
+    cta_teardown(c, ok);
+}
+
+constexpr int kAdamThreads = 128;
+constexpr int kAdamLoads = 37;        // slots read at once: the 148 of a training step in four rounds
+static_assert(kParams % kAdamThreads == 0, "whole blocks, and one for the loss");
+
+// Sum of p[0], p[stride], ... in that order, kAdamLoads loads in flight.
+__device__ __forceinline__ float slot_sum(const float* __restrict__ p, size_t stride, int n) {
+    float s = 0.0f;
+    for (int k = 0; k < n; k += kAdamLoads) {
+        float v[kAdamLoads];
+#pragma unroll
+        for (int i = 0; i < kAdamLoads; ++i) v[i] = k + i < n ? __ldg(p + (size_t)(k + i) * stride) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < kAdamLoads; ++i)
+            if (k + i < n) s += v[i];
+    }
+    return s;
 }
 
 // Adam over the summed gradient partials; writes f32 master weights and the
-// bf16 image.  Bias-corrected with beta^(step+1) from the control block.
-__global__ void k_mlp_adam(const float* __restrict__ partials, int n_parts, float* w, float* m, float* v,
-                           uint16_t* img, const TrainCtl* ctl, float lr, float b1, float b2, float eps) {
+// bf16 image; c1 and c2 are the bias corrections 1 - beta^(step+1).  The last
+// block sums the loss instead.  Bound by reading the slots (22 MB, from L2):
+// with one load after the other in flight, and the loss in a kernel of its
+// own, a step's end took 7.3 + 6.7 us, now 5.7 us together
+// (with 16 loads in flight 7.1, with 80 11.3).
+__global__ void __launch_bounds__(kAdamThreads)
+    k_mlp_adam(const float* __restrict__ partials, const double* __restrict__ loss_partials, int n_parts, float* w,
+               float* m, float* v, uint16_t* img, float c1, float c2, float lr, float b1, float b2, float eps,
+               double* history, double loss_norm) {
+    if (blockIdx.x == gridDim.x - 1) {
+        __shared__ double part[kAdamThreads];
+        if (!history) return;
+        double s = 0.0;
+        for (int k0 = 0; k0 < n_parts; k0 += kAdamThreads) {
+            if (k0 + (int)threadIdx.x < n_parts) part[threadIdx.x] = loss_partials[k0 + threadIdx.x];
+            __syncthreads();
+            if (threadIdx.x == 0)
+                for (int k = 0; k < min(kAdamThreads, n_parts - k0); ++k) s += part[k];
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) *history = s * loss_norm;
+        return;
+    }
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= kParams) return;
     if (padded_param(p)) return;
-    float g = 0.0f;
-    for (int k = 0; k < n_parts; ++k) g += partials[(size_t)k * kParams + p];
+    const float g = slot_sum(partials + p, kParams, n_parts);
     const float mm = b1 * m[p] + (1.0f - b1) * g;
     const float vv = b2 * v[p] + (1.0f - b2) * g * g;
     m[p] = mm;
     v[p] = vv;
-    const float mh = mm / (float)(1.0 - ctl->b1t);
-    const float vh = vv / (float)(1.0 - ctl->b2t);
+    const float mh = mm / c1;
+    const float vh = vv / c2;
     const float nw = w[p] - lr * mh / (sqrtf(vh) + eps);
     w[p] = nw;
     __nv_bfloat16 h = __float2bfloat16_rn(nw);
     img[image_offset(p) / 2] = *reinterpret_cast<uint16_t*>(&h);
-}
-
-__global__ void k_mlp_step_end(TrainCtl* ctl, const double* loss_partials, int n_parts, double* history,
-                               int64_t history_len, double loss_norm, float b1, float b2) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0.0;
-    for (int k = 0; k < n_parts; ++k) s += loss_partials[k];
-    const unsigned long long st = ctl->step;
-    if (history && (int64_t)st < history_len) history[st] = s * loss_norm;
-    ctl->step = st + 1;
-    ctl->b1t *= b1;
-    ctl->b2t *= b2;
 }
 
 // f32 master weights -> bf16 image
@@ -567,46 +671,87 @@ __global__ void k_mlp_pack(const float* __restrict__ w, uint16_t* img) {
 __global__ void k_grad_sum(const float* __restrict__ partials, int n_parts, float* g) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= kParams) return;
-    float s = 0.0f;
-    for (int k = 0; k < n_parts; ++k) s += partials[(size_t)k * kParams + p];
-    g[p] = s;
+    g[p] = slot_sum(partials + p, kParams, n_parts);
 }
 
-// forward pass: scaled outputs (explicit samples) or the predicted state
+// forward pass: scaled outputs (explicit samples) or the predicted state.
+// Layer 4 of a tile and layer 1 of the next one share a stage, and the samples
+// are read while MMAs work: three stages and three epilogues per tile.  120,000
+// cells: 29.7 us (33.6 with four stages, each waited for by all).
 __global__ void __launch_bounds__(kThreads, 1) k_mlp_forward(const ForwardArgs a, int64_t n_tiles) {
     extern __shared__ __align__(1024) uint8_t sm[];
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bar[2];
     __shared__ uint32_t slot;
     Cta c;
-    cta_setup(c, sm, a.img, &bar, &slot, a.ctl);
-    bool ok = true;
-    for (int64_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        float f[8], tg[5];
-        bool valid = false;
-        if (c.group == 0) {
-            valid = load_sample(a.s, tile, 0, c.row, f, tg);
-            put_x(c.sm, c.row, valid, f);
-        }
-        if (!(ok = forward(c))) break;
-        if (c.group != 0) continue;
-        float y[16];
-        umma::ld16(c.tm + kTmS2 + c.lane, y);
-        if (!valid) continue;
-        const int64_t i = tile * kTile + c.row;
-        if (a.y) {
-#pragma unroll
-            for (int k = 0; k < kOutputs; ++k) a.y[i * kOutputs + k] = y[k];
-        } else {
-            float q[kOutputs];
-#pragma unroll
-            for (int k = 0; k < kOutputs; ++k) q[k] = fmaf(a.scale[k], y[k], a.qinf[k]);
-            const float4 ru = make_float4(q[1], q[2], q[3], 0.0f);
-            a.rho0[i] = q[0]; a.rho1[i] = q[0];
-            a.rhou0[i] = ru; a.rhou1[i] = ru;
-            a.rhoe0[i] = q[4]; a.rhoe1[i] = q[4];
-        }
+    cta_setup(c, sm, a.img, bar, &slot, a.ctl);
+    const uint32_t A1 = c.sa + kSmA1, A2 = c.sa + kSmA2, A3 = c.sa + kSmA3;
+    const uint32_t W1 = c.sa + kImgW1, W2 = c.sa + kImgW2, W3 = c.sa + kImgW3, W4 = c.sa + kImgW4;
+    const uint32_t S1 = c.tm + kTmS1, S2 = c.tm + kTmS2;
+    const bool rowwork = c.group == 0;
+    float f[8], tg[5];
+    bool valid = false;
+    if (rowwork) {
+        valid = load_sample(a.s, blockIdx.x, 0, c.row, f, tg);
+        put_x(c.sm + kSmX, c.row, valid, f);
     }
-    cta_teardown(c, a.ctl, ok, 9);
+    auto layer1 = [&](int x) { gemm(S1, c.sa + kSmX + x * kXBytes, kIn, false, W1, kIn, false, 128, kHid, kIn, false); };
+    bool ok = stage(c, 9, [&] {
+        layer1(0);
+        umma::commit(c.bar);
+    });
+    int x = 0;
+    for (int64_t tile = blockIdx.x; ok && tile < n_tiles; tile += gridDim.x) {
+        const int64_t next = tile + gridDim.x;
+        bool valid_next = false;
+        epi_silu(c, kTmS1, c.sm + kSmA1);
+        if (!(ok = stage(
+                  c, 9,
+                  [&] {
+                      gemm(S1, A1, kHid, false, W2, kHid, false, 128, kHid, kHid, false);
+                      umma::commit(c.bar);
+                  },
+                  [&] { if (rowwork && next < n_tiles) valid_next = load_sample(a.s, next, 0, c.row, f, tg); })))
+            break;
+        epi_silu(c, kTmS1, c.sm + kSmA2);
+        if (!(ok = stage(
+                  c, 9,
+                  [&] {
+                      gemm(S1, A2, kHid, false, W3, kHid, false, 128, kHid, kHid, false);
+                      umma::commit(c.bar);
+                  },
+                  [&] { if (rowwork && next < n_tiles) put_x(c.sm + kSmX + (x ^ 1) * kXBytes, c.row, valid_next, f); })))
+            break;
+        epi_silu(c, kTmS1, c.sm + kSmA3);
+        x ^= 1;
+        if (!(ok = stage(c, 9, [&] {
+                  gemm(S2, A3, kHid, false, W4, kHid, false, 128, kOutPad, kHid, false);
+                  if (next < n_tiles) layer1(x);
+                  umma::commit(c.bar);
+              })))
+            break;
+        if (rowwork) {
+            float y[16];
+            umma::ld16(S2 + c.lane, y);
+            if (valid) {
+                const int64_t i = tile * kTile + c.row;
+                if (a.y) {
+#pragma unroll
+                    for (int k = 0; k < kOutputs; ++k) a.y[i * kOutputs + k] = y[k];
+                } else {
+                    float q[kOutputs];
+#pragma unroll
+                    for (int k = 0; k < kOutputs; ++k) q[k] = fmaf(a.scale[k], y[k], a.qinf[k]);
+                    const float4 ru = make_float4(q[1], q[2], q[3], 0.0f);
+                    a.rho0[i] = q[0]; a.rho1[i] = q[0];
+                    a.rhou0[i] = ru; a.rhou1[i] = ru;
+                    a.rhoe0[i] = q[4]; a.rhoe1[i] = q[4];
+                }
+            }
+        }
+        valid = valid_next;
+    }
+    ok = !__syncthreads_or(!ok || c.failed);
+    cta_teardown(c, ok);
 }
 
 // ---- features ----
@@ -757,7 +902,7 @@ bool set_smem_attrs() {
     if (done) return true;
     if (!ok_(cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmBytes),
              "warm start kernel attributes") ||
-        !ok_(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmBytes),
+        !ok_(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmForward),
              "warm start kernel attributes"))
         return false;
     done = true;
@@ -794,7 +939,7 @@ bool check_ctl(WS* w, cudaStream_t s, const char* what) {
 
 bool reset_ctl(WS* w, cudaStream_t s) {
     // through the pinned copy: every user of it has ended its stream (check_ctl)
-    *w->h_ctl = TrainCtl{0ull, 0.9, 0.999, 0, w->wait_cycles};
+    *w->h_ctl = TrainCtl{0, w->wait_cycles};
     return ok_(cudaMemcpyAsync(w->d_ctl, w->h_ctl, sizeof(TrainCtl), cudaMemcpyHostToDevice, s), "warm start control");
 }
 
@@ -832,7 +977,7 @@ bool forward_launch(WS* w, const ForwardArgs& fa, int64_t n_tiles, cudaStream_t 
     if (n_tiles <= 0) return true;
     if (!set_smem_attrs()) return false;
     const int grid = (int)std::min<int64_t>(n_tiles, n_sms());
-    k_mlp_forward<<<grid, kThreads, kSmBytes, s>>>(fa, n_tiles);
+    k_mlp_forward<<<grid, kThreads, kSmForward, s>>>(fa, n_tiles);
     count_launch();
     return ok_(cudaGetLastError(), "warm start forward");
 }
@@ -1143,19 +1288,21 @@ int64_t gbWarmStartTrain(gbWarmStart* w, int epochs, int tiles_per_cta, float lr
     ta.dy_scale = 2.0f / (float)(per_step * kTile * kOutputs);
     const double loss_norm = 1.0 / (double)(per_step * kTile * kOutputs);
     const int64_t hist_len = d_hist ? std::min(history_len, n_steps) : 0;
-    auto enqueue_step = [&](cudaStream_t st) {
-        k_mlp_train<<<grid, kThreads, kSmBytes, st>>>(ta);
-        k_mlp_adam<<<(kParams + 255) / 256, 256, 0, st>>>(d_partials, grid, w->d_w, w->d_m, w->d_v, w->d_img,
-                                                           w->d_ctl, lr, 0.9f, 0.999f, 1e-8f);
-        k_mlp_step_end<<<1, 32, 0, st>>>(w->d_ctl, d_lossp, grid, d_hist, hist_len, loss_norm, 0.9f, 0.999f);
-    };
-    // Launched one by one: a step takes about 100 us on the device and its
-    // three launches 6 us on the host, so a graph of 64 steps only added its
-    // own making (0.7 ms per training).
+    const float b1 = 0.9f, b2 = 0.999f;
+    double b1t = 0.9, b2t = 0.999;       // beta^(step + 1)
+    // Launched one by one: a step takes about 80 us on the device and its two
+    // launches 4 us on the host, so a graph of 64 steps only added its own
+    // making (0.7 ms per training).
     int64_t done = 0;
     while (ok && done < n_steps) {
-        enqueue_step(s);
-        count_launch(3);
+        ta.step = done;
+        k_mlp_train<<<grid, kThreads, kSmBytes, s>>>(ta);
+        k_mlp_adam<<<kParams / kAdamThreads + 1, kAdamThreads, 0, s>>>(
+            d_partials, d_lossp, grid, w->d_w, w->d_m, w->d_v, w->d_img, (float)(1.0 - b1t), (float)(1.0 - b2t), lr, b1,
+            b2, 1e-8f, done < hist_len ? d_hist + done : nullptr, loss_norm);
+        count_launch(2);
+        b1t *= b1;
+        b2t *= b2;
         ++done;
         ok = ok_(cudaGetLastError(), "gbWarmStartTrain");
         if (ok && done % 4096 == 0) ok = check_ctl(w, s, "gbWarmStartTrain");
