@@ -1,16 +1,18 @@
 // Batched multi-instance Euler solver: many (mesh, Mach, AoA) instances on
 // meshes of uneven sizes advanced together.
 //
-// Each iteration is four kernels that each cover every active instance --
-// boundary ghosts, gradients + limiters, flux + update, and a
+// Where the instances fit on the GPU together, one cell per thread, a run is
+// the batched persistent loop (euler_loop.cu).  Otherwise an iteration is
+// three kernels that each cover every active instance -- gradients + limiters
+// with the boundary conditions applied inside, flux + update, and a
 // per-instance residual reduction that also flips the instance's value
 // buffer and freezes it once its residual ratio drops below the tolerance --
 // captured in a CUDA graph and replayed.  Work is a list of (instance, tile
 // of cells) items, one block each; the list holds the active instances only
 // (it is rebuilt when instances freeze), and its order (the "schedule") and
-// the tile size are picked by an autotuner.  In tile-major order the instances that share a mesh process
-// the same tile back to back, so the mesh data of that tile is read from HBM
-// once and reused from L2 by the other instances.
+// the tile size are picked by an autotuner.  In tile-major order the instances
+// that share a mesh process the same tile back to back, so the mesh data of
+// that tile is read from HBM once and reused from L2 by the other instances.
 //
 // The per-cell arithmetic is the single-mesh path's (euler_ops.cuh), summed
 // in the same order; the residual of each instance is reduced in a fixed
@@ -20,7 +22,7 @@
 #include <string>
 #include <vector>
 
-#include "euler_ops.cuh"
+#include "euler_loop.cuh"
 #include "gb_internal.h"
 
 namespace gb {
@@ -470,6 +472,18 @@ struct gbBatchImpl {
     bool inject_barrier_fault = false;
     std::vector<void*> allocations;
     std::string signature;
+    // the batched loop (euler_loop.cu), made at its first use
+    struct {
+        int threads = -1;                     // -1: not looked at yet, 0: does not apply
+        int blocks = 0, faces = 4;
+        std::vector<gb::BatchLoopInst> h_inst;
+        gb::BatchLoopInst* d_inst = nullptr;
+        int* d_inst_of_block = nullptr;
+        gb::TagRec* recs = nullptr;
+        size_t n_recs = 0;
+        unsigned int tag = 0;                 // next unused tag; 0: the records are not cleared
+        gb::RunCtl* ctl = nullptr;
+    } loop;
 };
 
 namespace gb {
@@ -657,6 +671,147 @@ void enqueue_iteration(Batch* b, float cfl, double tol, cudaStream_t s) {
     k_batch_reduce<<<b->n_inst, kBlock, 0, s>>>(b->d_inst, tol);
 }
 
+// What the batched loop needs, if the instances fit on the GPU together one
+// cell per thread.  False: the kernels of an iteration run instead (nothing
+// is left in the error state).
+bool ensure_batch_loop(Batch* b) {
+    auto& L = b->loop;
+    if (L.threads >= 0) return L.threads > 0;
+    L.threads = 0;
+    int64_t chunks = 0;
+    std::vector<int64_t> of(b->n_inst);
+    for (int i = 0; i < b->n_inst; ++i) {
+        const MeshAccess& A = b->acc[b->h_inst[i].mesh];
+        if (A.N == 0) return false;
+        L.faces = std::max(L.faces, (int)A.dev->max_faces);
+        of[i] = (A.N + 31) / 32;
+        chunks += of[i];
+    }
+    // one block more per instance: its reducer
+    const int64_t room = (int64_t)kLoopBlocksPerSM * sm_count() - b->n_inst;
+    if (room <= 0 || chunks > room * (kLoopFull / 32)) return false;
+    int threads = (int)std::max<int64_t>(64, (chunks + room - 1) / room * 32);
+    auto blocks_at = [&](int t) {
+        int64_t n = 0;
+        for (int64_t c : of) n += (c + t / 32 - 1) / (t / 32);
+        return n;
+    };
+    while (threads <= kLoopFull && blocks_at(threads) > room) threads += 32;
+    if (threads > kLoopFull || loop_lean(L.faces, threads) || loop_smem(L.faces, threads) > kLoopSmem) return false;
+    L.blocks = (int)blocks_at(threads) + b->n_inst;
+    struct Quiet {
+        bool ok = false;
+        ~Quiet() {
+            if (ok) return;
+            clear_error();
+            cudaGetLastError();
+        }
+    } quiet;
+    cudaStream_t s = (cudaStream_t)gbGetStream();
+    std::vector<float4*> off(b->meshes.size(), nullptr);
+    const char* what = "batch loop";
+    for (size_t m = 0; m < b->meshes.size(); ++m) {
+        if (!balloc(b, off[m], (size_t)b->acc[m].G, what)) return false;
+        launch_ghost_off(*b->acc[m].dev, off[m], s);
+    }
+    L.n_recs = 0;
+    for (int i = 0; i < b->n_inst; ++i) {
+        const MeshAccess& A = b->acc[b->h_inst[i].mesh];
+        L.n_recs += 4 * (size_t)A.N + 2 * (size_t)A.dev->S + (size_t)of[i] + 1;
+    }
+    if (!balloc(b, L.recs, L.n_recs, what) || !balloc(b, L.ctl, 1, what) || !balloc(b, L.d_inst, b->n_inst, what) ||
+        !balloc(b, L.d_inst_of_block, L.blocks, what))
+        return false;
+    std::vector<int> inst_of_block;
+    L.h_inst.assign(b->n_inst, BatchLoopInst{});
+    TagRec* r = L.recs;
+    for (int i = 0; i < b->n_inst; ++i) {
+        const InstDev& I = b->h_inst[i];
+        const MeshAccess& A = b->acc[I.mesh];
+        const size_t N = (size_t)A.N;
+        BatchLoopInst& a = L.h_inst[i];
+        a.N = (uint32_t)N;
+        a.ctl = L.ctl;
+        a.n_groups = (int)((A.N + kBlock - 1) / kBlock);
+        a.n_blocks = (int)((of[i] + threads / 32 - 1) / (threads / 32));
+        a.first_block = (int)inst_of_block.size();
+        inst_of_block.insert(inst_of_block.end(), a.n_blocks + 1, i);
+        a.m = mesh_dev(*A.dev);
+        a.ghost_off = off[I.mesh];
+        for (int k = 0; k < 2; ++k) {
+            a.rho[k] = I.rho[k];
+            a.rhou[k] = I.rhou[k];
+            a.rhoe[k] = I.rhoe[k];
+            a.state[k] = r + 2 * N * k;
+        }
+        a.rec = r + 4 * N;
+        a.wsum = a.rec + 2 * (size_t)A.dev->S;
+        a.verdict = reinterpret_cast<unsigned long long*>(a.wsum + of[i]);
+        r = a.wsum + of[i] + 1;
+        a.rec_rho = I.rec_rho;
+        a.rec_rhou = I.rec_rhou;
+        a.ghosts.n = A.n_regions;
+        for (int k = 0; k <= A.n_regions; ++k) a.ghosts.start[k] = A.region_start[k];
+        for (int k = 0; k < A.n_regions; ++k) {
+            a.ghosts.type[k] = -1;
+            if (I.bc[k] < 0) continue;
+            const BcDev& c = b->h_bcs[I.bc[k]];
+            a.ghosts.type[k] = c.type;
+            a.ghosts.mach[k] = c.mach;
+            a.ghosts.p[k] = c.p;
+            a.ghosts.temp[k] = c.t;
+        }
+        InstDev* D = b->d_inst + i;
+        a.cur = &D->cur;
+        a.status = &D->status;
+        a.n_iters = &D->iters;
+        a.res0 = &D->res0;
+        a.ratio = &D->ratio;
+    }
+    if (!ok_(cudaMemcpyAsync(L.d_inst_of_block, inst_of_block.data(), inst_of_block.size() * sizeof(int),
+                             cudaMemcpyHostToDevice, s), what) ||
+        !ok_(cudaStreamSynchronize(s), what))
+        return false;
+    L.threads = threads;
+    quiet.ok = true;
+    return true;
+}
+
+// One launch of the batched loop for `iters` iterations of every active
+// instance (h_inst is up to date); false also when one of its waits gave up.
+bool launch_loop(Batch* b, float cfl, double tol, int iters, cudaStream_t s) {
+    auto& L = b->loop;
+    const char* what = "batch loop";
+    // no record of an earlier launch carries a tag of this one
+    if (L.tag == 0 || L.tag > (1u << 31)) {
+        if (!ok_(cudaMemsetAsync(L.recs, 0, L.n_recs * sizeof(TagRec), s), what)) return false;
+        L.tag = 1;
+    }
+    for (int i = 0; i < b->n_inst; ++i) {
+        const InstDev& I = b->h_inst[i];
+        BatchLoopInst& a = L.h_inst[i];
+        a.iters = I.status == 0 ? iters : 0;
+        a.cur0 = I.cur;
+        a.tol = tol;
+        a.tag0 = L.tag;
+        a.cfl = cfl;
+        a.max_iter = I.max_iter;
+        a.res0_fixed = I.res0_fixed;
+        a.history = I.hist;
+    }
+    L.tag += (unsigned int)iters + 1u;
+    int err = 0;
+    const bool ok =
+        ok_(cudaMemsetAsync(L.ctl, 0, sizeof(RunCtl), s), what) &&
+        ok_(cudaMemcpyAsync(L.d_inst, L.h_inst.data(), L.h_inst.size() * sizeof(BatchLoopInst), cudaMemcpyHostToDevice,
+                            s), what) &&
+        ok_(launch_batch_loop(L.d_inst, L.d_inst_of_block, L.blocks, L.faces, L.threads, reference_momentum(), s), what) &&
+        ok_(cudaMemcpyAsync(&err, &L.ctl->error, sizeof(int), cudaMemcpyDeviceToHost, s), what) &&
+        ok_(cudaStreamSynchronize(s), what);
+    if (ok && err) set_error("batch: a wait of the persistent loop gave up");
+    return ok && err == 0;
+}
+
 // Cells per work item while only some instances are still iterating: the
 // tuned tile, halved (down to 256) until the active instances give at least
 // 4 items per SM, so that a last slow instance still spreads over the GPU.
@@ -700,14 +855,26 @@ int64_t run_loop(Batch* b, float cfl, int64_t max_iter, double tol, int check_ev
         return good;
     };
     const bool persistent = b->variant >= kPersistentVariant;
-    ok = ok && build_items(b) && (persistent || capture());
+    // The batched loop in place of the default form's kernels (with its tile
+    // the residual's sums are the same too), where the instances fit and a
+    // launch pays for loading the geometry.  Measured per iteration against
+    // the graph, us (B200): 100 iterations of 2 x 4,608 prisms 11.4 / 21.0, 10
+    // instances of 57,168 together 15.7 / 23.1, 1 x 50,000 12.7 / 23.0, 1 x
+    // 120,000 18.6 / 36.6; 4 iterations a launch 29.5 / 35.6, 33.9 / 37.4, 30.1 /
+    // 37.2, and 9 of the 120,000 30.5 / 40.3.
+    const int64_t chunk0 = std::min<int64_t>(check_every, max_iter);
+    const bool loop = b->variant == 0 && b->tile == kBlock && chunk0 >= 4 && ensure_batch_loop(b) &&
+                      chunk0 >= (b->loop.threads <= kLoopWide ? 4 : 8);
+    ok = ok && (loop || (build_items(b) && (persistent || capture())));
     const int tuned = b->tile;
     int64_t done = 0;
     int active = b->n_inst;
     while (ok && done < max_iter) {
         const int64_t chunk = std::min<int64_t>(check_every, max_iter - done);
         b->table_stale = true;
-        if (persistent) {
+        if (loop) {
+            ok = launch_loop(b, cfl, tol, (int)chunk, s);
+        } else if (persistent) {
             ok = launch_persistent(b, cfl, tol, (int)chunk, s) && persistent_ok(b, s);
         } else {
             const int per_iter = 1 + (b->n_cell_items ? 2 : 0);
@@ -721,7 +888,7 @@ int64_t run_loop(Batch* b, float cfl, int64_t max_iter, double tol, int check_ev
         int now = 0;
         for (const InstDev& I : b->h_inst) now += I.status == 0;
         if (now == 0) break;
-        if (now != active) {             // drop the frozen instances' work
+        if (!loop && now != active) {    // drop the frozen instances' work
             active = now;
             const int t = active_tile(b, tuned);
             if (t != b->tile) {
@@ -968,10 +1135,17 @@ int gbBatchAutotune(gbBatch* b, gb_scalar cfl, int trial_iters, int* tile_out, i
             b->variant = c.variant;
             reset_counters(b, 1 << 30, false);
             ok = ok && size_partials(b) && build_items(b) && upload_inst(b);
-            // one untimed iteration, then the timed trial
-            if (ok) enqueue_iteration(b, cfl, 0.0, s);
+            // one untimed iteration (or launch of the loop, where a run would take it), then the timed trial
+            const bool loop = ok && c.variant == 0 && c.tile == kBlock && iters >= 4 && ensure_batch_loop(b);
+            if (loop) {
+                b->table_stale = true;
+                ok = launch_loop(b, cfl, 0.0, 4, s) && download_inst(b);
+            } else if (ok) {
+                enqueue_iteration(b, cfl, 0.0, s);
+            }
             cudaEventRecord(e0, s);
-            if (b->variant >= kPersistentVariant) ok = ok && launch_persistent(b, cfl, 0.0, iters, s);
+            if (loop) ok = ok && launch_loop(b, cfl, 0.0, iters, s);
+            else if (b->variant >= kPersistentVariant) ok = ok && launch_persistent(b, cfl, 0.0, iters, s);
             else for (int it = 0; it < iters && ok; ++it) enqueue_iteration(b, cfl, 0.0, s);
             cudaEventRecord(e1, s);
             ok = ok && ok_(cudaEventSynchronize(e1), "gbBatchAutotune");

@@ -36,8 +36,21 @@ constexpr int loop_smem(int max_faces, int threads) {
     return loop_smem_of(max_faces, threads, loop_lean(max_faces, threads));
 }
 
+// One instance of a batch in the batched loop: its own workers and reducer,
+// and what k_batch_reduce keeps of it.
+struct BatchLoopInst : EulerLoopArgs {
+    int first_block;                      // workers [first_block, first_block + n_blocks), then the reducer
+    int max_iter;
+    double res0_fixed;
+    int *cur, *status, *n_iters;
+    double *res0, *ratio, *history;       // history may be null
+};
+
 void launch_ghost_off(const DevMesh& d, float4* ghost_off, cudaStream_t s);
 cudaError_t launch_euler_loop(EulerLoopArgs& a, int max_faces, int threads, bool transposed, cudaStream_t s);
+// blocks: of the grid; inst_of_block: the instance of each.  threads <= kLoopFull.
+cudaError_t launch_batch_loop(const BatchLoopInst* insts, const int* inst_of_block, int blocks, int max_faces,
+                              int threads, bool transposed, cudaStream_t s);
 
 MeshDev mesh_dev(const DevMesh& m);
 
