@@ -128,8 +128,10 @@ __device__ __forceinline__ BatchGhostBcs batch_ghosts(BatchBcShared& sh, const I
 // Four forms of the batched iteration: variant 0 and 1 are two register
 // budgets of the gradient / flux kernels (resident 256-thread blocks per SM;
 // 1 trades a few spills for one more resident block), variant 2 runs the
-// gradient pass in 64-thread blocks that stage each cell's per-face entries
-// in shared memory with cp.async (flux as in variant 1), and variants 3 and 4
+// gradient pass in 128-thread blocks, a cell per thread, that stage each cell's
+// per-face entries in shared memory with cp.async (flux as in variant 1; 64
+// threads with several cells each, one after the other, took 41 to 62 us where
+// this takes 21 to 54, and the same on full GPUs), and variants 3 and 4
 // are the persistent kernel (k_batch_persistent), which runs a whole chunk of
 // iterations in one cooperative launch, budgeted for 4 or 3 resident
 // 256-thread blocks per SM.  The autotuner picks one.
@@ -137,8 +139,12 @@ constexpr int kBatchGradBlocks[2] = {4, 5};
 constexpr int kBatchFluxBlocks[2] = {4, 5};
 constexpr int kBatchVariants = 5;
 constexpr int kPersistentVariant = 3;     // 3 and 4
-constexpr int kStagedThreads = 64;
-constexpr int kStagedBlocks = 14;
+constexpr int kStagedThreads = 128;       // divides kBlock
+// Cells from which variant 0 takes the staged gradient pass too.  us per
+// iteration, from global memory / staged (B200): 4 x 50,000 prisms 41.6 / 43.9,
+// 300,000 73.5 / 72.5, 10 x 50,000 102.9 / 92.8, 8 x 120,000 185 / 163, 64
+// instances of 8.9 million together 1,410 / 1,231.
+constexpr int64_t kStagedCells = 300000;
 
 template <bool TRANSPOSED, int BLOCKS>
 __global__ void __launch_bounds__(kBlock, BLOCKS)
@@ -160,39 +166,37 @@ __global__ void __launch_bounds__(kBlock, BLOCKS)
         grad_lim_cell<TRANSPOSED>(m, q, g, i, __ldg(&m.nfc[i]), EntriesGlobal{m, i}, gh);
 }
 
-template <bool TRANSPOSED>
-__global__ void __launch_bounds__(kStagedThreads, kStagedBlocks)
+// MAXF: shared-memory slots per thread, at least the meshes' most faces per cell
+template <bool TRANSPOSED, int MAXF>
+__global__ void __launch_bounds__(kStagedThreads, MAXF <= 5 ? 8 : 7)
     k_batch_grad_staged(const int2* __restrict__ items, const InstDev* insts, const MeshTab* __restrict__ meshes,
                         int tile, const BcDev* __restrict__ bcs) {
     constexpr int B = kStagedThreads;
-    __shared__ float4 s_dn[kSlots * B], s_df[kSlots * B];
-    __shared__ uint32_t s_nbc[kSlots * B];
+    __shared__ float4 s_dn[MAXF * B], s_df[MAXF * B];
+    __shared__ uint32_t s_nbc[MAXF * B];
     __shared__ BatchBcShared s_bc;
-    const int2 w = items[blockIdx.x];
+    const uint32_t parts = (uint32_t)tile / B;
+    const int2 w = items[blockIdx.x / parts];
     const InstDev& I = insts[w.x];
     if (I.status) return;                      // uniform over the block
     const MeshTab& M = meshes[I.mesh];
     const MeshDev m = M.m;
+    const uint32_t tid = threadIdx.x, c0 = (uint32_t)w.y * tile + blockIdx.x % parts * B, i = c0 + tid;
+    if (c0 >= m.N) return;                     // uniform too
     const BatchGhostBcs gh = batch_ghosts(s_bc, I, M, bcs);
+    if (i >= m.N) return;
     const int cur = I.cur;
     const EulerState q{I.rho[cur], I.rhou[cur], I.rhoe[cur]};
     const EulerGrad g{nullptr, nullptr, nullptr, I.rec_rho, I.rec_rhou};
-    const uint32_t c0 = (uint32_t)w.y * tile;
-    const uint32_t c1 = min(m.N, c0 + (uint32_t)tile);
-    const uint32_t tid = threadIdx.x;
-    // the slots are this thread's own; the previous cell's reads of them have
-    // completed before its results were stored
-    for (uint32_t i = c0 + tid; i < c1; i += B) {
-        const uint32_t nf = __ldg(&m.nfc[i]);
-        for (uint32_t t = 0; t < nf; ++t) {
-            const uint32_t k = i + t * m.N;
-            cp_async4(&s_nbc[t * B + tid], &m.nbc[k]);
-            cp_async16(&s_dn[t * B + tid], &m.dn[k]);
-            cp_async16(&s_df[t * B + tid], &m.df[k]);
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        grad_lim_cell<TRANSPOSED>(m, q, g, i, nf, EntriesStaged<B>{s_nbc + tid, s_dn + tid, s_df + tid}, gh);
+    const uint32_t nf = __ldg(&m.nfc[i]);
+    for (uint32_t t = 0; t < nf; ++t) {
+        const uint32_t k = i + t * m.N;
+        cp_async4(&s_nbc[t * B + tid], &m.nbc[k]);
+        cp_async16(&s_dn[t * B + tid], &m.dn[k]);
+        cp_async16(&s_df[t * B + tid], &m.df[k]);
     }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    grad_lim_cell<TRANSPOSED>(m, q, g, i, nf, EntriesStaged<B>{s_nbc + tid, s_dn + tid, s_df + tid}, gh);
 }
 
 template <int BLOCKS>
@@ -645,6 +649,15 @@ bool persistent_ok(Batch* b, cudaStream_t s) {
     return err == 0;
 }
 
+template <bool TRANSPOSED>
+void launch_grad_staged(Batch* b, cudaStream_t s) {
+    int faces = 0;
+    for (const MeshAccess& A : b->acc) faces = std::max(faces, (int)A.dev->max_faces);
+    const int n = b->n_cell_items * (b->tile / kStagedThreads);
+    if (faces <= 5) k_batch_grad_staged<TRANSPOSED, 5><<<n, kStagedThreads, 0, s>>>(b->d_cell_items, b->d_inst, b->d_mesh, b->tile, b->d_bcs);
+    else k_batch_grad_staged<TRANSPOSED, kSlots><<<n, kStagedThreads, 0, s>>>(b->d_cell_items, b->d_inst, b->d_mesh, b->tile, b->d_bcs);
+}
+
 void enqueue_iteration(Batch* b, float cfl, double tol, cudaStream_t s) {
     if (b->variant >= kPersistentVariant) {
         launch_persistent(b, cfl, tol, 1, s);
@@ -654,19 +667,18 @@ void enqueue_iteration(Batch* b, float cfl, double tol, cudaStream_t s) {
     if (b->n_cell_items) {
         const int n = b->n_cell_items;
         const bool tr = reference_momentum();
-        if (b->variant == 0) {
+        if (b->variant == 2 || (b->variant == 0 && (int64_t)n * b->tile >= kStagedCells)) {
+            if (tr) launch_grad_staged<true>(b, s);
+            else launch_grad_staged<false>(b, s);
+        } else if (b->variant == 0) {
             if (tr) k_batch_grad<true, kBatchGradBlocks[0]><<<n, kBlock, 0, s>>>(b->d_cell_items, b->d_inst, b->d_mesh, b->tile, b->d_bcs);
             else k_batch_grad<false, kBatchGradBlocks[0]><<<n, kBlock, 0, s>>>(b->d_cell_items, b->d_inst, b->d_mesh, b->tile, b->d_bcs);
-            k_batch_flux<kBatchFluxBlocks[0]><<<n, kBlock, 0, s>>>(b->d_cell_items, b->d_inst, b->d_mesh, b->tile, cfl);
-        } else if (b->variant == 1) {
+        } else {
             if (tr) k_batch_grad<true, kBatchGradBlocks[1]><<<n, kBlock, 0, s>>>(b->d_cell_items, b->d_inst, b->d_mesh, b->tile, b->d_bcs);
             else k_batch_grad<false, kBatchGradBlocks[1]><<<n, kBlock, 0, s>>>(b->d_cell_items, b->d_inst, b->d_mesh, b->tile, b->d_bcs);
-            k_batch_flux<kBatchFluxBlocks[1]><<<n, kBlock, 0, s>>>(b->d_cell_items, b->d_inst, b->d_mesh, b->tile, cfl);
-        } else {
-            if (tr) k_batch_grad_staged<true><<<n, kStagedThreads, 0, s>>>(b->d_cell_items, b->d_inst, b->d_mesh, b->tile, b->d_bcs);
-            else k_batch_grad_staged<false><<<n, kStagedThreads, 0, s>>>(b->d_cell_items, b->d_inst, b->d_mesh, b->tile, b->d_bcs);
-            k_batch_flux<kBatchFluxBlocks[1]><<<n, kBlock, 0, s>>>(b->d_cell_items, b->d_inst, b->d_mesh, b->tile, cfl);
         }
+        if (b->variant == 0) k_batch_flux<kBatchFluxBlocks[0]><<<n, kBlock, 0, s>>>(b->d_cell_items, b->d_inst, b->d_mesh, b->tile, cfl);
+        else k_batch_flux<kBatchFluxBlocks[1]><<<n, kBlock, 0, s>>>(b->d_cell_items, b->d_inst, b->d_mesh, b->tile, cfl);
     }
     k_batch_reduce<<<b->n_inst, kBlock, 0, s>>>(b->d_inst, tol);
 }

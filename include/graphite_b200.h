@@ -339,7 +339,10 @@ int gbBatchGetState(gbBatch* batch, int instance, float* rho, float* rhou, float
  * order + 2 * kernel variant (schedule 0..9); order 0 runs instance by
  * instance, 1 tile by tile across the instances of a mesh; variant 0 / 1
  * compiles the gradient and flux kernels for 4 / 5 resident 256-thread blocks
- * per SM, variant 2 runs the gradient pass in 64-thread blocks that stage
+ * per SM (variant 0 stages the entries as variant 2 does from 300,000 active
+ * cells, and with 256-cell tiles runs as one persistent launch per check_every
+ * iterations where the instances fit on the GPU one cell per thread), variant 2
+ * runs the gradient pass in 128-thread blocks that stage
  * each cell's face entries in shared memory (flux as variant 1), variants 3
  * and 4 are one persistent cooperative kernel per check_every iterations
  * (the three phases of an iteration separated by grid-wide barriers), with 4

@@ -106,3 +106,24 @@ def test_batch_loop_stops_and_options(case_of, kw):
     assert same(kernels, loop) == []
     if "bad" in kw:
         assert loop[3][kw["bad"]] == 3
+
+
+@pytest.mark.parametrize("make,regions,n", [
+    (lambda: meshgen.airfoil_2d_prisms(500, 148), WING, 2),           # 296,000 cells: below the line
+    (lambda: meshgen.airfoil_2d_prisms(500, 151), WING, 2),           # 302,000: staged, five slots
+    (lambda: meshgen.channel_bump(62, 41, 61, cells="hex"), DUCT, 2),  # staged, six slots
+])
+def test_default_form_of_large_batches_is_bitwise_the_unstaged_one(tmp_path, make, regions, n):
+    p = str(tmp_path / "m.su2")
+    make().write_su2(p)
+    c = EulerCase(p)
+    out = []
+    for tuning in ((256, 1), (256, 3), (512, 4)):
+        with EulerBatch([c], [(0, bcs(regions, 0.4 + 0.1 * i)) for i in range(n)]) as b:
+            b.set_tuning(*tuning)
+            for i in range(n):
+                b.init_uniform(i, (0.4 + 0.1 * i, 0.0, 0.02), P, T)
+            b.run(0.5, 12)
+            out.append([x for i in range(n) for x in b.get_state(i)])
+    c.close()
+    assert same(out[0], out[1]) == [] and same(out[0], out[2]) == []
