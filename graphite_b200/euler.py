@@ -4,8 +4,8 @@
 the reference's entry points -- load the mesh, create rho/rhou/rhoe/error,
 initialise from a free stream, and per iteration apply the boundary
 conditions, prepare gradients and limiters, step, and reduce the residual --
-but calls libgraphite_b200.so.  ``run`` uses the graph-replayed loop
-(gbEulerRun) instead of one C call per stage.
+but calls libgraphite_b200.so.  ``run`` uses the whole loop of
+gbEulerRun instead of one C call per stage.
 
 Boundary conditions are tuples ``("slip", region)`` or
 ``("farfield", region, mach_x, mach_y, mach_z, pressure, temperature)``.
@@ -150,7 +150,7 @@ class EulerCase:
         return arr
 
     def run(self, bcs, cfl: float, n_iter: int, tolerance: float = 0.0, check_every: int = 100) -> np.ndarray:
-        """n_iter iterations as replayed CUDA graphs; returns the residual
+        """n_iter iterations as persistent launches or replayed CUDA graphs; returns the residual
         history (stops early below ``tolerance`` relative to the first)."""
         arr = self.bc_structs(bcs)
         hist = np.zeros(max(n_iter, 1), dtype=np.float64)

@@ -2,7 +2,7 @@
 
 ``NSICase`` holds a mesh with "velocity" and "pressure" fields and runs the
 loop the reference's PhysicsNSI (src/models/nsi.cu) lays out -- boundary
-conditions, FvmNSIStepPrepare, FvmNSIStep, residual -- or the graph-replayed
+conditions, FvmNSIStepPrepare, FvmNSIStep, residual -- or the whole loop of
 gbNSIRun.  Boundary conditions are tuples ``("slip", region)``,
 ``("wall", region)`` (no-slip) or ``("inletoutlet", region, ux, uy, uz, p)``.
 """
