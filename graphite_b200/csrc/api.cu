@@ -135,6 +135,7 @@ struct MeshImpl {
     PendingBcs pending;
     RunGraphs euler_run, nsi_run;
     LoopPlan loop, nsi_loop;
+    unsigned int loop_polls = 0;      // limit of the persistent loops' waits, 0: the default
     Workspace ws;
     cudaStream_t capture = nullptr;   // stream the loops are captured on
     double* h_result = nullptr;       // pinned: FvmFieldReduceSum's value on the host
@@ -763,6 +764,7 @@ void loop_args(const MeshImpl* mi, const LoopPlan& lp, LoopArgs& a, double toler
     a.partials = partials;
     a.n_groups = (int)((mi->dev.N + kBlock - 1) / kBlock);
     a.n_blocks = lp.n_blocks;
+    a.spin0 = loop_spin_start(mi->loop_polls);
     a.wsum = lp.recs + lp.n_recs - 1 - 2 * warps;
     a.wsum_rho = a.wsum + warps;
     a.verdict = reinterpret_cast<unsigned long long*>(a.wsum_rho + warps);
@@ -1291,6 +1293,14 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
     if (residual_history && done > 0) memcpy(residual_history, hist.data(), (size_t)done * sizeof(double));
     if (density_history && done > 0) memcpy(density_history, hist_rho.data(), (size_t)done * sizeof(double));
     return done;
+}
+
+int gbMeshSetLoopWaitLimit(cuMesh* mesh, unsigned int polls) {
+    clear_error();
+    MeshImpl* mi = impl(mesh);
+    if (!mi) { set_error("gbMeshSetLoopWaitLimit: null mesh"); return 1; }
+    mi->loop_polls = polls;
+    return 0;
 }
 
 int64_t gbEulerRun(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* rhoe, FvmField* error, gb_scalar cfl,

@@ -487,6 +487,7 @@ struct gbBatchImpl {
         size_t n_recs = 0;
         unsigned int tag = 0;                 // next unused tag; 0: the records are not cleared
         gb::RunCtl* ctl = nullptr;
+        unsigned int polls = 0;               // limit of its waits, 0: the default
     } loop;
 };
 
@@ -806,6 +807,7 @@ bool launch_loop(Batch* b, float cfl, double tol, int iters, cudaStream_t s) {
         a.cur0 = I.cur;
         a.tol = tol;
         a.tag0 = L.tag;
+        a.spin0 = loop_spin_start(L.polls);
         a.cfl = cfl;
         a.max_iter = I.max_iter;
         a.res0_fixed = I.res0_fixed;
@@ -1093,6 +1095,13 @@ int gbBatchInjectBarrierFault(gbBatch* b) {
     clear_error();
     if (!b) { set_error("gbBatchInjectBarrierFault: null batch"); return 1; }
     b->inject_barrier_fault = true;
+    return 0;
+}
+
+int gbBatchSetLoopWaitLimit(gbBatch* b, unsigned int polls) {
+    clear_error();
+    if (!b) { set_error("gbBatchSetLoopWaitLimit: null batch"); return 1; }
+    b->loop.polls = polls;
     return 0;
 }
 

@@ -145,7 +145,7 @@ __device__ __forceinline__ bool grad_loop_cell(const EulerLoopArgs& a, int buf, 
 #pragma unroll
     for (int c = 0; c < 5; ++c) { gs[c] = make_float3(0.f, 0.f, 0.f); vmin[c] = v[c]; vmax[c] = v[c]; }
     int ng = 0;
-    Patience wait(&a.ctl->error);
+    Patience wait(a);
     auto add = [&](int t, float r, float4 ue) {
         const float3 d = g.dn3(t);
         const float w = WIDE ? g.w2(t) : 1.f / ydot(d, d);
@@ -297,7 +297,7 @@ template <int MAXF, bool WIDE, bool FULL, bool LEAN>
 __device__ __forceinline__ bool flux_loop_cell(const EulerLoopArgs& a, unsigned int tag, const TileGeo<MAXF, LEAN>& g,
                                                uint32_t i, int nf, FluxSum& s) {
     const MeshDev& m = a.m;
-    Patience wait(&a.ctl->error);
+    Patience wait(a);
     auto twin = [&](uint32_t word) { return &a.rec[(word >> 28) * m.N + (word & kNbMask)]; };
     if constexpr (WIDE) {
         float rb[MAXF];
@@ -443,7 +443,7 @@ __device__ void batch_reducer(const BatchLoopInst& a) {
     double res0 = *a.res0;
     for (int it = 0; it < a.iters; ++it) {
         const unsigned int tag = a.tag0 + it;
-        const double bs = reduce_groups(a.wsum, a.N, a.n_groups, tag, nullptr, &a.ctl->error, ok);
+        const double bs = reduce_groups(a, a.wsum, tag, nullptr, ok);
         if (!ok) return;
         if (n == 0) res0 = a.res0_fixed > 0.0 ? a.res0_fixed : bs;
         const double ratio = res0 > 0.0 ? bs / res0 : 0.0;

@@ -16,6 +16,13 @@ struct alignas(16) TagRec {
 // One cell per thread, two blocks per SM.
 constexpr int kLoopBlocksPerSM = 2;
 constexpr int kLoopSmem = 112 * 1024;   // dynamic shared memory of a block, at most
+// Polls of a wait before it gives up (a poll takes about half a microsecond).
+constexpr unsigned int kLoopSpinLimit = 1u << 23;
+
+// Where a wait of at most `polls` polls (0: the default) starts counting.
+constexpr unsigned int loop_spin_start(unsigned int polls) {
+    return polls == 0 || polls > kLoopSpinLimit ? 0u : kLoopSpinLimit - polls;
+}
 
 struct LoopArgs {
     uint32_t N;
@@ -27,14 +34,12 @@ struct LoopArgs {
     double *out, *partials;               // the residual, and its sums by 256-cell group
     int n_groups, n_blocks;
     unsigned int tag0;                    // tags of this launch: tag0 + iteration
+    unsigned int spin0;                   // loop_spin_start of the launch's limit
     TagRec *wsum, *wsum_rho;              // per warp: a double
     unsigned long long* verdict;          // tag of the last iteration judged (low word), halt (high word)
 };
 
 namespace {
-
-// Polls of a wait before it gives up (a poll takes about half a microsecond).
-constexpr unsigned int kLoopSpinLimit = 1u << 23;
 
 // A record is one 16-byte access only while all four of its words are used: a
 // load with dead words may be narrowed to several, which can then see two
@@ -68,11 +73,13 @@ __device__ __forceinline__ void st_relaxed64(unsigned long long* p, unsigned lon
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;\n" ::"l"(p), "l"(v) : "memory");
 }
 
-// Counts the polls of one wait; false once it, or another one, has given up.
+// Counts the polls of one wait up to kLoopSpinLimit; false once it, or another
+// one, has given up.  A shorter limit is a later start, so that the test of
+// every 256th poll is all there is either way.
 struct Patience {
-    unsigned int n = 0;
+    unsigned int n;
     int* error;
-    __device__ __forceinline__ explicit Patience(int* e) : error(e) {}
+    __device__ __forceinline__ explicit Patience(const LoopArgs& a) : n(a.spin0), error(&a.ctl->error) {}
     __device__ __forceinline__ bool more() {
         if ((++n & 255u) == 0u && (n >= kLoopSpinLimit || *(volatile int*)error)) {
             atomicExch(error, 1);
@@ -93,12 +100,12 @@ __device__ __forceinline__ double warp_sum(double x) {
 // (into `groups`), the groups strided over 256 (virtual) threads, then the
 // block tree.  Every thread of the block calls it and gets the sum; ok turns
 // false when a wait gave up.
-__device__ double reduce_groups(const TagRec* wsum, uint32_t N, int n_groups, unsigned int tag, double* groups,
-                                int* error, bool& ok) {
+__device__ double reduce_groups(const LoopArgs& a, const TagRec* wsum, unsigned int tag, double* groups, bool& ok) {
     __shared__ double sv[kBlock];
     __shared__ double sw[kBlock / 32];
-    const uint32_t n_warps = (N + 31) / 32;
-    Patience wait(error);
+    const uint32_t n_warps = (a.N + 31) / 32;
+    const int n_groups = a.n_groups;
+    Patience wait(a);
     for (int v = threadIdx.x; v < kBlock; v += blockDim.x) {
         double s = 0.0;
         for (int i = v; i < n_groups; i += kBlock) {
@@ -143,11 +150,11 @@ __device__ void loop_reducer(const LoopArgs& a) {
     bool ok = true;
     for (int it = 0; it < a.iters; ++it) {
         const unsigned int tag = a.tag0 + it;
-        const double bs = reduce_groups(a.wsum, a.N, a.n_groups, tag, nullptr, &ctl->error, ok);
+        const double bs = reduce_groups(a, a.wsum, tag, nullptr, ok);
         double rs = 0.0;
         if (a.hist_rho) {
             __syncthreads();
-            rs = reduce_groups(a.wsum_rho, a.N, a.n_groups, tag, nullptr, &ctl->error, ok);
+            rs = reduce_groups(a, a.wsum_rho, tag, nullptr, ok);
         }
         if (!ok) return;
         if (run0 + it == 0) res0 = bs;
@@ -157,7 +164,7 @@ __device__ void loop_reducer(const LoopArgs& a) {
         const bool last = halt || it + 1 == a.iters;
         if (last) {
             __syncthreads();
-            reduce_groups(a.wsum, a.N, a.n_groups, tag, a.partials, &ctl->error, ok);
+            reduce_groups(a, a.wsum, tag, a.partials, ok);
         }
         if (threadIdx.x == 0) {
             st_relaxed64(a.verdict, (unsigned long long)halt << 32 | tag);
@@ -181,7 +188,7 @@ __device__ void loop_reducer(const LoopArgs& a) {
 // Whether the update of iteration `tag` may happen: false when the iteration
 // before it has stopped the loop, or the wait for its verdict gave up.
 __device__ __forceinline__ bool await_verdict(const LoopArgs& a, unsigned int tag) {
-    Patience wait(&a.ctl->error);
+    Patience wait(a);
     for (;;) {
         const unsigned long long v = ld_relaxed64(a.verdict);
         if ((unsigned int)v >= tag - 1u) return (v >> 32) == 0;

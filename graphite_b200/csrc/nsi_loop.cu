@@ -129,7 +129,7 @@ __device__ __forceinline__ bool nsi_grad_cell(const NsiLoopArgs& a, const NsiGho
     float vmin[4], vmax[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) { gs[c] = make_float3(0.f, 0.f, 0.f); vmin[c] = v[c]; vmax[c] = v[c]; }
-    Patience wait(&a.ctl->error);
+    Patience wait(a);
     auto add = [&](int t, const NsiState& q) {
         const float3 d = g.dn3(t);
         const float w = g.w2(d);
@@ -202,7 +202,7 @@ __device__ __forceinline__ bool nsi_flux_cell(const NsiLoopArgs& a, const NsiGho
                                               const NsiGeo<MAXF, WIDE>& g, int buf, unsigned int tag, int nf,
                                               const NsiState& own, const float4 go[4], NsiSum& s) {
     const uint32_t N = a.N;
-    Patience wait(&a.ctl->error);
+    Patience wait(a);
 #pragma unroll 1
     for (int t = 0; t < nf; ++t) {
         const uint32_t word = g.nb(t), j = word & kNbMask;

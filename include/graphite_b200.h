@@ -295,6 +295,13 @@ int64_t gbEulerRun(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* rhoe, 
                    gb_scalar cfl, int64_t n_iter, const gbBc* bcs, int n_bc, double tolerance,
                    int check_every, double* residual_history);
 
+/* Bound, in polls of about half a microsecond, on each wait of this mesh's
+ * persistent launches (gbEulerRun, gbNSIRun; polls 0, or more than 2^23: the
+ * default, 2^23).  A wait that gives up makes the call return an error; the
+ * fields then hold states of different iterations, and the next call runs
+ * normally.  Tests set a tiny bound to exercise that path without a fault. */
+int gbMeshSetLoopWaitLimit(cuMesh* mesh, unsigned int polls);
+
 /* gbEulerRun that also writes, per iteration, the density part of the
  * residual, sum over cells of F_rho^2 V (float64, fixed order), to
  * density_history (host array of n_iter doubles; its square root relative
@@ -357,6 +364,8 @@ int gbBatchGetTuning(gbBatch* batch, int* tile_cells, int* schedule);
  * and the run returns an error instead of hanging; the launch after it runs
  * normally. */
 int gbBatchInjectBarrierFault(gbBatch* batch);
+/* gbMeshSetLoopWaitLimit for the persistent launches of schedules 0 and 1. */
+int gbBatchSetLoopWaitLimit(gbBatch* batch, unsigned int polls);
 
 /* Times trial_iters iterations of every (tile, schedule) candidate from the
  * current states (restored afterwards), then the 4 fastest again over
