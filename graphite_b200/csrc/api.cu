@@ -411,6 +411,7 @@ bool ensure_partials(FieldImpl* fi, int n) {
     if (fi->n_partials >= n) return true;
     dfree(fi->partials);
     fi->n_partials = 0;
+    fi->partials_valid = false;
     if (!dalloc(fi->partials, (size_t)n, "alloc partials")) return false;
     fi->n_partials = n;
     return true;
@@ -653,17 +654,25 @@ bool ensure_run_graphs(MeshImpl* mi, RunGraphs& rg, std::vector<uint64_t>& key, 
     return true;
 }
 
+// How a run of a loop ended.
+struct RunEnd {
+    int64_t ran = 0;          // iterations whose states and residuals are in the fields and histories
+    bool finished = false;    // false: a call failed or a wait gave up (an error): the fields hold no one iteration's data
+    bool diverged = false;    // the last residual is not finite (an error)
+    int64_t result() const { return finished && !diverged ? ran : -1; }
+};
+
 // Replays the graphs from value buffer `cur` for up to n_iter iterations,
 // check_every at a time.  The device stops iterating once a residual is
 // below tolerance x the run's first one (tolerance > 0) or is not finite;
 // after each chunk the iterations it actually ran come back to `hist`.
-// Returns the iterations run (the last one the first below tolerance, when
-// the tolerance is met), or -1 when a residual was not finite (an error);
-// `cur` becomes the buffer holding the last state.
-int64_t replay_run_graphs(RunGraphs& rg, int& cur, int64_t n_iter, int64_t check_every, std::vector<double>& hist,
+// The last iteration run is the first below tolerance, when the tolerance is
+// met; `cur` becomes the buffer holding the last state.
+RunEnd replay_run_graphs(RunGraphs& rg, int& cur, int64_t n_iter, int64_t check_every, std::vector<double>& hist,
                           cudaStream_t s, const char* what, std::vector<double>* hist2 = nullptr) {
     const int cur0 = cur;
     int64_t done = 0;
+    bool diverged = false;
     bool ok = cuda_ok(cudaMemsetAsync(rg.ctl, 0, sizeof(RunCtl), s), what);
     while (ok && done < n_iter) {
         const int64_t chunk = std::min<int64_t>(check_every, n_iter - done);
@@ -685,15 +694,12 @@ int64_t replay_run_graphs(RunGraphs& rg, int& cur, int64_t n_iter, int64_t check
         if (!ok) break;
         const int64_t ran = (int64_t)std::min<unsigned long long>(rg.h_ctl->it_chunk, (unsigned long long)chunk);
         done += ran;
-        if (rg.h_ctl->halt == 2) {
-            set_error(std::string(what) + ": residual is not finite (diverged)");
-            ok = false;
-            break;
-        }
+        diverged = rg.h_ctl->halt == 2;
+        if (diverged) set_error(std::string(what) + ": residual is not finite (diverged)");
         if (rg.h_ctl->halt != 0 || ran < chunk) break;
     }
     cur = (int)((cur0 + done) & 1);
-    return ok ? done : -1;
+    return RunEnd{done, ok, diverged};
 }
 
 int sm_count() {
@@ -773,9 +779,10 @@ size_t loop_tail_recs(const DevMesh& d) { return 2 * (((size_t)d.N + 31) / 32) +
 
 // Up to n_iter iterations, check_every to a launch; as replay_run_graphs.
 template <class Launch>
-int64_t run_loop(LoopPlan& lp, LoopArgs& a, Launch&& launch, int& cur, int64_t n_iter, int64_t check_every,
+RunEnd run_loop(LoopPlan& lp, LoopArgs& a, Launch&& launch, int& cur, int64_t n_iter, int64_t check_every,
                  std::vector<double>& hist, std::vector<double>* hist2, cudaStream_t s, const char* what) {
     int64_t done = 0;
+    bool diverged = false;
     bool ok = cuda_ok(cudaMemsetAsync(lp.ctl, 0, sizeof(RunCtl), s), what);
     while (ok && done < n_iter) {
         const int64_t chunk = std::min<int64_t>(std::min<int64_t>(check_every, n_iter - done), 1 << 20);
@@ -803,14 +810,12 @@ int64_t run_loop(LoopPlan& lp, LoopArgs& a, Launch&& launch, int& cur, int64_t n
         }
         const int64_t ran = (int64_t)std::min<unsigned long long>(lp.h_ctl->it_chunk, (unsigned long long)chunk);
         done += ran;
-        if (lp.h_ctl->halt == 2) {
-            set_error(std::string(what) + ": residual is not finite (diverged)");
-            ok = false;
-        }
-        if (!ok || lp.h_ctl->halt != 0 || ran < chunk) break;
+        diverged = lp.h_ctl->halt == 2;
+        if (diverged) set_error(std::string(what) + ": residual is not finite (diverged)");
+        if (lp.h_ctl->halt != 0 || ran < chunk) break;
     }
     cur = (int)((cur + done) & 1);
-    return ok ? done : -1;
+    return RunEnd{done, ok, diverged};
 }
 }  // namespace
 
@@ -1233,9 +1238,10 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
         a.cfl = cfl;
         int cur = impl(rho)->cur;
         std::vector<double> hist((size_t)n_iter, 0.0), hist_rho(density ? (size_t)n_iter : 0, 0.0);
-        const int64_t done = run_loop(
+        const RunEnd end = run_loop(
             lp, a, [&] { return launch_euler_loop(a, faces, lp.threads, transposed, s); }, cur, n_iter, check_every, hist,
             density ? &hist_rho : nullptr, s, "gbEulerRun");
+        const int64_t done = end.result();
         if (done > 0) {
             // what the kernels of an iteration leave behind: the ghost states of the last gradient pass, from the
             // state it read (the buffer before the last update), and its face states
@@ -1244,7 +1250,7 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
             if (!launch_ok("gbEulerRun")) return -1;
         }
         impl(rho)->cur = impl(rhou)->cur = impl(rhoe)->cur = cur;
-        ei->partials_valid = true;
+        ei->partials_valid = end.finished;   // else the residual is the sum of the field as it is
         if (residual_history && done > 0) memcpy(residual_history, hist.data(), (size_t)done * sizeof(double));
         if (density_history && done > 0) memcpy(density_history, hist_rho.data(), (size_t)done * sizeof(double));
         return done;
@@ -1280,8 +1286,9 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
         return -1;
     int cur = impl(rho)->cur;
     std::vector<double> hist((size_t)n_iter, 0.0), hist_rho(density ? (size_t)n_iter : 0, 0.0);
-    const int64_t done = replay_run_graphs(mi->euler_run, cur, n_iter, check_every, hist, s, "gbEulerRun",
-                                           density ? &hist_rho : nullptr);
+    const RunEnd end = replay_run_graphs(mi->euler_run, cur, n_iter, check_every, hist, s, "gbEulerRun",
+                                         density ? &hist_rho : nullptr);
+    const int64_t done = end.result();
     if (done > 0 && inline_bcs) {
         // the ghost states of the last gradient pass, from the state it read
         // (the buffer before the last update), into both value buffers
@@ -1289,7 +1296,7 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
         if (!launch_ok("gbEulerRun")) return -1;
     }
     impl(rho)->cur = impl(rhou)->cur = impl(rhoe)->cur = cur;
-    ei->partials_valid = true;
+    ei->partials_valid = end.finished;   // else the residual is the sum of the field as it is
     if (residual_history && done > 0) memcpy(residual_history, hist.data(), (size_t)done * sizeof(double));
     if (density_history && done > 0) memcpy(density_history, hist_rho.data(), (size_t)done * sizeof(double));
     return done;
@@ -1553,9 +1560,10 @@ int64_t gbNSIRun(cuMesh* mesh, FvmField* velocity, FvmField* pressure, FvmField*
         a.limited = t_nsi.limited;
         int cur = impl(pressure)->cur;
         std::vector<double> hist((size_t)n_iter, 0.0);
-        const int64_t done = run_loop(
+        const RunEnd end = run_loop(
             lp, a, [&] { return launch_nsi_loop(a, faces, lp.threads, s); }, cur, n_iter, check_every, hist, nullptr, s,
             "gbNSIRun");
+        const int64_t done = end.result();
         if (done > 0) {
             // what the kernels of an iteration leave behind: the ghost states and gradients of the state before the
             // last update
@@ -1569,7 +1577,7 @@ int64_t gbNSIRun(cuMesh* mesh, FvmField* velocity, FvmField* pressure, FvmField*
             if (!launch_ok("gbNSIRun")) return -1;
         }
         impl(velocity)->cur = impl(pressure)->cur = cur;
-        ei->partials_valid = true;
+        ei->partials_valid = end.finished;   // else the residual is the sum of the field as it is
         if (residual_history && done > 0) memcpy(residual_history, hist.data(), (size_t)done * sizeof(double));
         return done;
     }
@@ -1597,9 +1605,10 @@ int64_t gbNSIRun(cuMesh* mesh, FvmField* velocity, FvmField* pressure, FvmField*
         return -1;
     int cur = impl(pressure)->cur;
     std::vector<double> hist((size_t)n_iter, 0.0);
-    const int64_t done = replay_run_graphs(mi->nsi_run, cur, n_iter, check_every, hist, s, "gbNSIRun");
+    const RunEnd end = replay_run_graphs(mi->nsi_run, cur, n_iter, check_every, hist, s, "gbNSIRun");
+    const int64_t done = end.result();
     impl(velocity)->cur = impl(pressure)->cur = cur;
-    ei->partials_valid = true;
+    ei->partials_valid = end.finished;   // else the residual is the sum of the field as it is
     if (residual_history && done > 0) memcpy(residual_history, hist.data(), (size_t)done * sizeof(double));
     return done;
 }
