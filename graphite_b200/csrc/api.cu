@@ -1242,9 +1242,10 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
             lp, a, [&] { return launch_euler_loop(a, faces, lp.threads, transposed, s); }, cur, n_iter, check_every, hist,
             density ? &hist_rho : nullptr, s, "gbEulerRun");
         const int64_t done = end.result();
-        if (done > 0) {
-            // what the kernels of an iteration leave behind: the ghost states of the last gradient pass, from the
-            // state it read (the buffer before the last update), and its face states
+        if (end.finished && end.ran > 0) {
+            // what the kernels of an iteration leave behind, that of a residual that is not finite too: the ghost
+            // states of the last gradient pass, from the state it read (the buffer before the last update), and its
+            // face states
             launch_bc_table(mi->dev, gbt, 1 - cur, s);
             launch_grad_lim(mi->dev, state_of(rho, rhou, rhoe, 1 - cur), grad_of(rho, rhou, rhoe, false), transposed, s);
             if (!launch_ok("gbEulerRun")) return -1;
@@ -1289,7 +1290,7 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
     const RunEnd end = replay_run_graphs(mi->euler_run, cur, n_iter, check_every, hist, s, "gbEulerRun",
                                          density ? &hist_rho : nullptr);
     const int64_t done = end.result();
-    if (done > 0 && inline_bcs) {
+    if (end.finished && end.ran > 0 && inline_bcs) {
         // the ghost states of the last gradient pass, from the state it read
         // (the buffer before the last update), into both value buffers
         launch_bc_table(mi->dev, gbt, 1 - cur, s);
@@ -1564,9 +1565,9 @@ int64_t gbNSIRun(cuMesh* mesh, FvmField* velocity, FvmField* pressure, FvmField*
             lp, a, [&] { return launch_nsi_loop(a, faces, lp.threads, s); }, cur, n_iter, check_every, hist, nullptr, s,
             "gbNSIRun");
         const int64_t done = end.result();
-        if (done > 0) {
-            // what the kernels of an iteration leave behind: the ghost states and gradients of the state before the
-            // last update
+        if (end.finished && end.ran > 0) {
+            // what the kernels of an iteration leave behind, that of a residual that is not finite too: the ghost
+            // states and gradients of the state before the last update
             for (int r = 0; r < n_regions; ++r)
                 if (gt.type[r] >= 0)
                     enqueue_nsi_bc(mesh, velocity, pressure, r, gt.type[r], 1 - cur,

@@ -280,7 +280,8 @@ int gbApplyBoundaryConditions(cuMesh* mesh);
  * stops iterating there, although the host looks only every check_every
  * iterations (the iterations left in that chunk do nothing).  A residual
  * that is not finite stops it too, and the call returns -1 with "not finite"
- * in gbGetLastError().  Returns the number of iterations run, or -1 on
+ * in gbGetLastError(); the fields hold that iteration's state, as in the
+ * per-call loop.  Returns the number of iterations run, or -1 on
  * error.
  * The results, ghost values included, are bitwise those of the per-call
  * loop (FvmEuler*Bc, FvmEulerStepPrepare, FvmEulerStep, FvmFieldReduceSum);
