@@ -156,6 +156,8 @@ _PROTOS = {
     "gbBatchInjectBarrierFault": (C.c_int, [C.c_void_p]),
     "gbMeshSetLoopWaitLimit": (C.c_int, [MeshP, C.c_uint]),
     "gbBatchSetLoopWaitLimit": (C.c_int, [C.c_void_p, C.c_uint]),
+    "gbMeshInjectLoopRefusal": (C.c_int, [MeshP]),
+    "gbBatchInjectLoopRefusal": (C.c_int, [C.c_void_p]),
     "gbApplyBoundaryConditions": (C.c_int, [MeshP]),
     "gbBatchFree": (None, [C.c_void_p]),
     "gbBatchInitUniform": (C.c_int, [C.c_void_p, C.c_int, gb_vector, C.c_float, C.c_float]),

@@ -136,6 +136,7 @@ struct MeshImpl {
     RunGraphs euler_run, nsi_run;
     LoopPlan loop, nsi_loop;
     unsigned int loop_polls = 0;      // limit of the persistent loops' waits, 0: the default
+    bool refuse_loop = false;         // the next persistent launch counts as refused
     Workspace ws;
     cudaStream_t capture = nullptr;   // stream the loops are captured on
     double* h_result = nullptr;       // pinned: FvmFieldReduceSum's value on the host
@@ -659,6 +660,7 @@ struct RunEnd {
     int64_t ran = 0;          // iterations whose states and residuals are in the fields and histories
     bool finished = false;    // false: a call failed or a wait gave up (an error): the fields hold no one iteration's data
     bool diverged = false;    // the last residual is not finite (an error)
+    bool refused = false;     // the first launch was refused (no error is set): nothing has run
     int64_t result() const { return finished && !diverged ? ran : -1; }
 };
 
@@ -777,10 +779,14 @@ void loop_args(const MeshImpl* mi, const LoopPlan& lp, LoopArgs& a, double toler
 }
 size_t loop_tail_recs(const DevMesh& d) { return 2 * (((size_t)d.N + 31) / 32) + 1; }
 
-// Up to n_iter iterations, check_every to a launch; as replay_run_graphs.
+// Up to n_iter iterations, check_every to a launch; as replay_run_graphs.  A
+// cooperative launch is refused where its blocks do not fit on the GPU
+// together (a stream, process or device with fewer resources than the plan
+// was made for); the caller then replays the graphs.
 template <class Launch>
-RunEnd run_loop(LoopPlan& lp, LoopArgs& a, Launch&& launch, int& cur, int64_t n_iter, int64_t check_every,
-                 std::vector<double>& hist, std::vector<double>* hist2, cudaStream_t s, const char* what) {
+RunEnd run_loop(MeshImpl* mi, LoopPlan& lp, LoopArgs& a, Launch&& launch, int& cur, int64_t n_iter,
+                int64_t check_every, std::vector<double>& hist, std::vector<double>* hist2, cudaStream_t s,
+                const char* what) {
     int64_t done = 0;
     bool diverged = false;
     bool ok = cuda_ok(cudaMemsetAsync(lp.ctl, 0, sizeof(RunCtl), s), what);
@@ -795,7 +801,18 @@ RunEnd run_loop(LoopPlan& lp, LoopArgs& a, Launch&& launch, int& cur, int64_t n_
         }
         a.tag0 = lp.tag;
         lp.tag += (unsigned int)chunk + 1u;
-        ok = ok && cuda_ok(launch(), what) &&
+        const bool inject = mi->refuse_loop;
+        mi->refuse_loop = false;
+        const cudaError_t e = !ok ? cudaSuccess : inject ? cudaErrorCooperativeLaunchTooLarge : launch();
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            if (done == 0) {
+                RunEnd end;
+                end.refused = true;
+                return end;
+            }
+        }
+        ok = ok && cuda_ok(e, what) &&
              cuda_ok(cudaMemcpyAsync(hist.data() + done, lp.hist, (size_t)chunk * sizeof(double),
                                      cudaMemcpyDeviceToHost, s), what) &&
              (!hist2 || cuda_ok(cudaMemcpyAsync(hist2->data() + done, lp.hist + lp.cap, (size_t)chunk * sizeof(double),
@@ -1233,28 +1250,30 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
         a.rec_rhou = (float4*)impl(rhou)->rec;
         a.err = (float*)ei->val[ei->cur];
         a.ghost_off = lp.ghost_off;
-        gbt.store = 0;
         a.ghosts = gbt;
+        a.ghosts.store = 0;
         a.cfl = cfl;
         int cur = impl(rho)->cur;
         std::vector<double> hist((size_t)n_iter, 0.0), hist_rho(density ? (size_t)n_iter : 0, 0.0);
         const RunEnd end = run_loop(
-            lp, a, [&] { return launch_euler_loop(a, faces, lp.threads, transposed, s); }, cur, n_iter, check_every, hist,
+            mi, lp, a, [&] { return launch_euler_loop(a, faces, lp.threads, transposed, s); }, cur, n_iter, check_every, hist,
             density ? &hist_rho : nullptr, s, "gbEulerRun");
         const int64_t done = end.result();
-        if (end.finished && end.ran > 0) {
-            // what the kernels of an iteration leave behind, that of a residual that is not finite too: the ghost
-            // states of the last gradient pass, from the state it read (the buffer before the last update), and its
-            // face states
-            launch_bc_table(mi->dev, gbt, 1 - cur, s);
-            launch_grad_lim(mi->dev, state_of(rho, rhou, rhoe, 1 - cur), grad_of(rho, rhou, rhoe, false), transposed, s);
-            if (!launch_ok("gbEulerRun")) return -1;
+        if (!end.refused) {
+            if (end.finished && end.ran > 0) {
+                // what the kernels of an iteration leave behind, that of a residual that is not finite too: the ghost
+                // states of the last gradient pass, from the state it read (the buffer before the last update), and its
+                // face states
+                launch_bc_table(mi->dev, a.ghosts, 1 - cur, s);
+                launch_grad_lim(mi->dev, state_of(rho, rhou, rhoe, 1 - cur), grad_of(rho, rhou, rhoe, false), transposed, s);
+                if (!launch_ok("gbEulerRun")) return -1;
+            }
+            impl(rho)->cur = impl(rhou)->cur = impl(rhoe)->cur = cur;
+            ei->partials_valid = end.finished;   // else the residual is the sum of the field as it is
+            if (residual_history && done > 0) memcpy(residual_history, hist.data(), (size_t)done * sizeof(double));
+            if (density_history && done > 0) memcpy(density_history, hist_rho.data(), (size_t)done * sizeof(double));
+            return done;
         }
-        impl(rho)->cur = impl(rhou)->cur = impl(rhoe)->cur = cur;
-        ei->partials_valid = end.finished;   // else the residual is the sum of the field as it is
-        if (residual_history && done > 0) memcpy(residual_history, hist.data(), (size_t)done * sizeof(double));
-        if (density_history && done > 0) memcpy(density_history, hist_rho.data(), (size_t)done * sizeof(double));
-        return done;
     }
     // what the captured launches bake in
     std::vector<uint64_t> key;
@@ -1308,6 +1327,14 @@ int gbMeshSetLoopWaitLimit(cuMesh* mesh, unsigned int polls) {
     MeshImpl* mi = impl(mesh);
     if (!mi) { set_error("gbMeshSetLoopWaitLimit: null mesh"); return 1; }
     mi->loop_polls = polls;
+    return 0;
+}
+
+int gbMeshInjectLoopRefusal(cuMesh* mesh) {
+    clear_error();
+    MeshImpl* mi = impl(mesh);
+    if (!mi) { set_error("gbMeshInjectLoopRefusal: null mesh"); return 1; }
+    mi->refuse_loop = true;
     return 0;
 }
 
@@ -1562,25 +1589,27 @@ int64_t gbNSIRun(cuMesh* mesh, FvmField* velocity, FvmField* pressure, FvmField*
         int cur = impl(pressure)->cur;
         std::vector<double> hist((size_t)n_iter, 0.0);
         const RunEnd end = run_loop(
-            lp, a, [&] { return launch_nsi_loop(a, faces, lp.threads, s); }, cur, n_iter, check_every, hist, nullptr, s,
+            mi, lp, a, [&] { return launch_nsi_loop(a, faces, lp.threads, s); }, cur, n_iter, check_every, hist, nullptr, s,
             "gbNSIRun");
         const int64_t done = end.result();
-        if (end.finished && end.ran > 0) {
-            // what the kernels of an iteration leave behind, that of a residual that is not finite too: the ghost
-            // states and gradients of the state before the last update
-            for (int r = 0; r < n_regions; ++r)
-                if (gt.type[r] >= 0)
-                    enqueue_nsi_bc(mesh, velocity, pressure, r, gt.type[r], 1 - cur,
-                                   gb_vector{gt.vinf[r].x, gt.vinf[r].y, gt.vinf[r].z}, gt.pinf[r], s);
-            launch_nsi_grad(mi->dev, (const float*)impl(pressure)->val[1 - cur],
-                            (const float4*)impl(velocity)->val[1 - cur], impl(pressure)->grad, impl(velocity)->grad,
-                            t_nsi.limited, s);
-            if (!launch_ok("gbNSIRun")) return -1;
+        if (!end.refused) {
+            if (end.finished && end.ran > 0) {
+                // what the kernels of an iteration leave behind, that of a residual that is not finite too: the ghost
+                // states and gradients of the state before the last update
+                for (int r = 0; r < n_regions; ++r)
+                    if (gt.type[r] >= 0)
+                        enqueue_nsi_bc(mesh, velocity, pressure, r, gt.type[r], 1 - cur,
+                                       gb_vector{gt.vinf[r].x, gt.vinf[r].y, gt.vinf[r].z}, gt.pinf[r], s);
+                launch_nsi_grad(mi->dev, (const float*)impl(pressure)->val[1 - cur],
+                                (const float4*)impl(velocity)->val[1 - cur], impl(pressure)->grad, impl(velocity)->grad,
+                                t_nsi.limited, s);
+                if (!launch_ok("gbNSIRun")) return -1;
+            }
+            impl(velocity)->cur = impl(pressure)->cur = cur;
+            ei->partials_valid = end.finished;   // else the residual is the sum of the field as it is
+            if (residual_history && done > 0) memcpy(residual_history, hist.data(), (size_t)done * sizeof(double));
+            return done;
         }
-        impl(velocity)->cur = impl(pressure)->cur = cur;
-        ei->partials_valid = end.finished;   // else the residual is the sum of the field as it is
-        if (residual_history && done > 0) memcpy(residual_history, hist.data(), (size_t)done * sizeof(double));
-        return done;
     }
     std::vector<uint64_t> key;
     for (const FvmField* f : {velocity, pressure, error}) key_field(key, f);

@@ -488,6 +488,7 @@ struct gbBatchImpl {
         unsigned int tag = 0;                 // next unused tag; 0: the records are not cleared
         gb::RunCtl* ctl = nullptr;
         unsigned int polls = 0;               // limit of its waits, 0: the default
+        bool refuse = false;                  // the next launch counts as refused
     } loop;
 };
 
@@ -791,8 +792,10 @@ bool ensure_batch_loop(Batch* b) {
 }
 
 // One launch of the batched loop for `iters` iterations of every active
-// instance (h_inst is up to date); false also when one of its waits gave up.
-bool launch_loop(Batch* b, float cfl, double tol, int iters, cudaStream_t s) {
+// instance (h_inst is up to date); false also when one of its waits gave up,
+// and, with no error set, when the launch was refused (its blocks do not fit
+// on the GPU together) and `refused` is there to say so.
+bool launch_loop(Batch* b, float cfl, double tol, int iters, cudaStream_t s, bool* refused = nullptr) {
     auto& L = b->loop;
     const char* what = "batch loop";
     // no record of an earlier launch carries a tag of this one
@@ -814,14 +817,22 @@ bool launch_loop(Batch* b, float cfl, double tol, int iters, cudaStream_t s) {
         a.history = I.hist;
     }
     L.tag += (unsigned int)iters + 1u;
+    if (!ok_(cudaMemsetAsync(L.ctl, 0, sizeof(RunCtl), s), what) ||
+        !ok_(cudaMemcpyAsync(L.d_inst, L.h_inst.data(), L.h_inst.size() * sizeof(BatchLoopInst), cudaMemcpyHostToDevice,
+                             s), what))
+        return false;
+    const cudaError_t e = L.refuse ? cudaErrorCooperativeLaunchTooLarge
+                                   : launch_batch_loop(L.d_inst, L.d_inst_of_block, L.blocks, L.faces, L.threads,
+                                                       reference_momentum(), s);
+    L.refuse = false;
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        if (refused) *refused = true;
+        return refused ? false : ok_(e, what);
+    }
     int err = 0;
-    const bool ok =
-        ok_(cudaMemsetAsync(L.ctl, 0, sizeof(RunCtl), s), what) &&
-        ok_(cudaMemcpyAsync(L.d_inst, L.h_inst.data(), L.h_inst.size() * sizeof(BatchLoopInst), cudaMemcpyHostToDevice,
-                            s), what) &&
-        ok_(launch_batch_loop(L.d_inst, L.d_inst_of_block, L.blocks, L.faces, L.threads, reference_momentum(), s), what) &&
-        ok_(cudaMemcpyAsync(&err, &L.ctl->error, sizeof(int), cudaMemcpyDeviceToHost, s), what) &&
-        ok_(cudaStreamSynchronize(s), what);
+    const bool ok = ok_(cudaMemcpyAsync(&err, &L.ctl->error, sizeof(int), cudaMemcpyDeviceToHost, s), what) &&
+                    ok_(cudaStreamSynchronize(s), what);
     if (ok && err) set_error("batch: a wait of the persistent loop gave up");
     return ok && err == 0;
 }
@@ -877,8 +888,8 @@ int64_t run_loop(Batch* b, float cfl, int64_t max_iter, double tol, int check_ev
     // 120,000 18.6 / 36.6; 4 iterations a launch 29.5 / 35.6, 33.9 / 37.4, 30.1 /
     // 37.2, and 9 of the 120,000 30.5 / 40.3.
     const int64_t chunk0 = std::min<int64_t>(check_every, max_iter);
-    const bool loop = b->variant == 0 && b->tile == kBlock && chunk0 >= 4 && ensure_batch_loop(b) &&
-                      chunk0 >= (b->loop.threads <= kLoopWide ? 4 : 8);
+    bool loop = b->variant == 0 && b->tile == kBlock && chunk0 >= 4 && ensure_batch_loop(b) &&
+                chunk0 >= (b->loop.threads <= kLoopWide ? 4 : 8);
     ok = ok && (loop || (build_items(b) && (persistent || capture())));
     const int tuned = b->tile;
     int64_t done = 0;
@@ -887,7 +898,13 @@ int64_t run_loop(Batch* b, float cfl, int64_t max_iter, double tol, int check_ev
         const int64_t chunk = std::min<int64_t>(check_every, max_iter - done);
         b->table_stale = true;
         if (loop) {
-            ok = launch_loop(b, cfl, tol, (int)chunk, s);
+            bool refused = false;
+            ok = launch_loop(b, cfl, tol, (int)chunk, s, done == 0 ? &refused : nullptr);
+            if (refused) {                   // nothing has run: the kernels of an iteration instead
+                loop = false;
+                ok = build_items(b) && capture();
+                continue;
+            }
         } else if (persistent) {
             ok = launch_persistent(b, cfl, tol, (int)chunk, s) && persistent_ok(b, s);
         } else {
@@ -1105,6 +1122,13 @@ int gbBatchSetLoopWaitLimit(gbBatch* b, unsigned int polls) {
     return 0;
 }
 
+int gbBatchInjectLoopRefusal(gbBatch* b) {
+    clear_error();
+    if (!b) { set_error("gbBatchInjectLoopRefusal: null batch"); return 1; }
+    b->loop.refuse = true;
+    return 0;
+}
+
 int gbBatchGetTuning(gbBatch* b, int* tile_cells, int* schedule) {
     if (!b) return 1;
     if (tile_cells) *tile_cells = b->tile;
@@ -1157,13 +1181,15 @@ int gbBatchAutotune(gbBatch* b, gb_scalar cfl, int trial_iters, int* tile_out, i
             reset_counters(b, 1 << 30, false);
             ok = ok && size_partials(b) && build_items(b) && upload_inst(b);
             // one untimed iteration (or launch of the loop, where a run would take it), then the timed trial
-            const bool loop = ok && c.variant == 0 && c.tile == kBlock && iters >= 4 && ensure_batch_loop(b);
+            bool loop = ok && c.variant == 0 && c.tile == kBlock && iters >= 4 && ensure_batch_loop(b);
             if (loop) {
+                bool refused = false;
                 b->table_stale = true;
-                ok = launch_loop(b, cfl, 0.0, 4, s) && download_inst(b);
-            } else if (ok) {
-                enqueue_iteration(b, cfl, 0.0, s);
+                ok = launch_loop(b, cfl, 0.0, 4, s, &refused);
+                if (refused) ok = !(loop = false);
+                ok = ok && download_inst(b);
             }
+            if (ok && !loop) enqueue_iteration(b, cfl, 0.0, s);
             cudaEventRecord(e0, s);
             if (loop) ok = ok && launch_loop(b, cfl, 0.0, iters, s);
             else if (b->variant >= kPersistentVariant) ok = ok && launch_persistent(b, cfl, 0.0, iters, s);

@@ -508,8 +508,9 @@ cudaError_t launch(EulerLoopArgs& a, int threads, cudaStream_t s) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     void* args[] = {(void*)&a};
-    count_launch();
-    return cudaLaunchCooperativeKernel(fn, dim3(a.n_blocks + 1), dim3(threads), args, smem, s);
+    const cudaError_t r = cudaLaunchCooperativeKernel(fn, dim3(a.n_blocks + 1), dim3(threads), args, smem, s);
+    if (r == cudaSuccess) count_launch();
+    return r;
 }
 
 template <bool TRANSPOSED, int MAXF>
@@ -520,8 +521,9 @@ cudaError_t launch_batch(const BatchLoopInst* insts, const int* inst_of_block, i
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     void* args[] = {(void*)&insts, (void*)&inst_of_block};
-    count_launch();
-    return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(threads), args, smem, s);
+    const cudaError_t r = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(threads), args, smem, s);
+    if (r == cudaSuccess) count_launch();
+    return r;
 }
 
 }  // namespace

@@ -319,8 +319,9 @@ cudaError_t launch(NsiLoopArgs& a, int threads, cudaStream_t s) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     void* args[] = {(void*)&a};
-    count_launch();
-    return cudaLaunchCooperativeKernel(fn, dim3(a.n_blocks + 1), dim3(threads), args, smem, s);
+    const cudaError_t r = cudaLaunchCooperativeKernel(fn, dim3(a.n_blocks + 1), dim3(threads), args, smem, s);
+    if (r == cudaSuccess) count_launch();
+    return r;
 }
 
 }  // namespace

@@ -302,6 +302,10 @@ int64_t gbEulerRun(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* rhoe, 
  * fields then hold states of different iterations, and the next call runs
  * normally.  Tests set a tiny bound to exercise that path without a fault. */
 int gbMeshSetLoopWaitLimit(cuMesh* mesh, unsigned int polls);
+/* Test hook: the next persistent launch on this mesh counts as refused, as
+ * the driver refuses one whose blocks do not fit on the GPU together; the run
+ * replays its graphs instead, with the same results. */
+int gbMeshInjectLoopRefusal(cuMesh* mesh);
 
 /* gbEulerRun that also writes, per iteration, the density part of the
  * residual, sum over cells of F_rho^2 V (float64, fixed order), to
@@ -367,6 +371,8 @@ int gbBatchGetTuning(gbBatch* batch, int* tile_cells, int* schedule);
 int gbBatchInjectBarrierFault(gbBatch* batch);
 /* gbMeshSetLoopWaitLimit for the persistent launches of schedules 0 and 1. */
 int gbBatchSetLoopWaitLimit(gbBatch* batch, unsigned int polls);
+/* gbMeshInjectLoopRefusal for the next persistent launch of schedules 0 and 1. */
+int gbBatchInjectLoopRefusal(gbBatch* batch);
 
 /* Times trial_iters iterations of every (tile, schedule) candidate from the
  * current states (restored afterwards), then the 4 fastest again over
