@@ -135,6 +135,7 @@ struct MeshImpl {
     PendingBcs pending;
     RunGraphs euler_run, nsi_run;
     LoopPlan loop, nsi_loop;
+    std::atomic<float> sectors{-1.f}; // mesh_sectors, once counted
     unsigned int loop_polls = 0;      // limit of the persistent loops' waits, 0: the default
     bool refuse_loop = false;         // the next persistent launch counts as refused
     Workspace ws;
@@ -852,6 +853,12 @@ Workspace::~Workspace() {
     if (host) cudaFreeHost(host);
 }
 
+float mesh_sectors(cuMesh* mesh) {
+    MeshImpl* mi = impl(mesh);
+    if (mi->sectors < 0.f) mi->sectors = neighbour_sectors(mi->num);
+    return mi->sectors;
+}
+
 bool mesh_access(cuMesh* mesh, MeshAccess* out) {
     MeshImpl* mi = impl(mesh);
     if (!mi) { set_error("null mesh"); return false; }
@@ -1223,17 +1230,15 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
         }
     }
     const bool transposed = g_transposed.load() != 0;
-    // The persistent loop where the mesh fits on the GPU one cell per thread and
-    // a launch is long enough to pay for loading the cells' geometry.  Measured
-    // against the graphs, us per call of n iterations (B200): 4,608 prisms n = 2
-    // 78 / 81, n = 20 248 / 375; 50,000 prisms n = 2 82 / 82, n = 20 292 / 450;
-    // 120,000 prisms n = 5 181 / 180, n = 20 474 / 602; 140,736 prisms n = 10
-    // 351 / 336, n = 20 627 / 632, n = 300 29.1 / 30.0 per iteration.
+    // The persistent loop where the mesh fits on the GPU one cell per thread,
+    // its form is the faster one there and a launch is long enough to pay for
+    // loading the cells' geometry (loop_shape.h).
     const int threads = loop_threads(mi->dev), faces = std::max(mi->dev.max_faces, 4);
     const int64_t chunk = std::min<int64_t>(check_every, n_iter);
-    const int64_t shortest = threads <= kLoopWide ? 4 : (loop_lean(faces, threads) ? 32 : 8);
+    const LoopForm form = loop_form(faces, threads);
     const size_t N = (size_t)mi->dev.N, n_recs = 4 * N + 2 * (size_t)mi->dev.S + loop_tail_recs(mi->dev);
-    if (table_bcs && threads <= kLoopMax && loop_smem(faces, threads) <= kLoopSmem && chunk >= shortest &&
+    if (table_bcs && form != LoopForm::kNone && chunk >= 4 &&
+        chunk >= loop_shortest(form, faces, threads, mesh_sectors(mesh), false, n_iter) &&
         ensure_loop_plan(mi, mi->loop, threads, n_recs, chunk, "gbEulerRun")) {
         LoopPlan& lp = mi->loop;
         EulerLoopArgs a{};
@@ -1256,8 +1261,8 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
         int cur = impl(rho)->cur;
         std::vector<double> hist((size_t)n_iter, 0.0), hist_rho(density ? (size_t)n_iter : 0, 0.0);
         const RunEnd end = run_loop(
-            mi, lp, a, [&] { return launch_euler_loop(a, faces, lp.threads, transposed, s); }, cur, n_iter, check_every, hist,
-            density ? &hist_rho : nullptr, s, "gbEulerRun");
+            mi, lp, a, [&] { return launch_euler_loop(a, form, faces, lp.threads, transposed, s); }, cur, n_iter, check_every,
+            hist, density ? &hist_rho : nullptr, s, "gbEulerRun");
         const int64_t done = end.result();
         if (!end.refused) {
             if (end.finished && end.ran > 0) {
@@ -1559,17 +1564,13 @@ int64_t gbNSIRun(cuMesh* mesh, FvmField* velocity, FvmField* pressure, FvmField*
             gt.u[k] = (float4*)impl(velocity)->val[k];
         }
     }
-    // The persistent loop where the mesh fits on the GPU one cell per thread
-    // and a launch pays for loading the cells' geometry (as in euler_run).
-    // Measured per iteration against the graphs, us (B200): 1,152 hexes 7.4 /
-    // 19.9, 28,800 tets 8.3 / 26.6, 60,000 hexes 10.4 / 24.1, 100,000 hexes
-    // 20.1 / 29.1, with the limiter 1,152 hexes 15.1 / 24.0, 110,000 hexes 30.5
-    // / 32.1.
+    // The persistent loop under the same conditions as in euler_run.
     const int threads = loop_threads(mi->dev), faces = std::max(mi->dev.max_faces, 4);
     const int64_t chunk = std::min<int64_t>(check_every, n_iter);
     const size_t N = (size_t)mi->dev.N, n_recs = (4 + kNsiGradRecs) * N + loop_tail_recs(mi->dev);
     if (n_regions > 0 && n_regions <= kMaxNsiRegions && threads <= kNsiMax &&
-        nsi_loop_smem(faces, threads) <= kLoopSmem && chunk >= (threads <= kNsiWide ? 4 : 8) &&
+        nsi_loop_smem(faces, threads) <= kLoopSmem && chunk >= 4 &&
+        chunk >= nsi_loop_shortest(faces, threads, mesh_sectors(mesh), t_nsi.limited != 0, inline_bcs, n_iter) &&
         ensure_loop_plan(mi, mi->nsi_loop, threads, n_recs, chunk, "gbNSIRun")) {
         LoopPlan& lp = mi->nsi_loop;
         NsiLoopArgs a{};

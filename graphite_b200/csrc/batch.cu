@@ -480,6 +480,8 @@ struct gbBatchImpl {
     struct {
         int threads = -1;                     // -1: not looked at yet, 0: does not apply
         int blocks = 0, faces = 4;
+        float sectors = 0.f;                  // mesh_sectors, mean over the instances' cells
+        gb::LoopForm form = gb::LoopForm::kNone;
         std::vector<gb::BatchLoopInst> h_inst;
         gb::BatchLoopInst* d_inst = nullptr;
         int* d_inst_of_block = nullptr;
@@ -693,6 +695,7 @@ bool ensure_batch_loop(Batch* b) {
     if (L.threads >= 0) return L.threads > 0;
     L.threads = 0;
     int64_t chunks = 0;
+    double sectors = 0.0;
     std::vector<int64_t> of(b->n_inst);
     for (int i = 0; i < b->n_inst; ++i) {
         const MeshAccess& A = b->acc[b->h_inst[i].mesh];
@@ -700,7 +703,9 @@ bool ensure_batch_loop(Batch* b) {
         L.faces = std::max(L.faces, (int)A.dev->max_faces);
         of[i] = (A.N + 31) / 32;
         chunks += of[i];
+        sectors += (double)of[i] * mesh_sectors(b->meshes[b->h_inst[i].mesh]);
     }
+    L.sectors = (float)(sectors / (double)std::max<int64_t>(chunks, 1));
     // one block more per instance: its reducer
     const int64_t room = (int64_t)kLoopBlocksPerSM * sm_count() - b->n_inst;
     if (room <= 0 || chunks > room * (kLoopFull / 32)) return false;
@@ -711,7 +716,9 @@ bool ensure_batch_loop(Batch* b) {
         return n;
     };
     while (threads <= kLoopFull && blocks_at(threads) > room) threads += 32;
-    if (threads > kLoopFull || loop_lean(L.faces, threads) || loop_smem(L.faces, threads) > kLoopSmem) return false;
+    L.form = loop_form(L.faces, threads);
+    if (L.form != LoopForm::kWide && L.form != LoopForm::kNarrow) return false;
+    if (loop_shortest(L.form, L.faces, threads, L.sectors, true, 0) == kLoopNever) return false;
     L.blocks = (int)blocks_at(threads) + b->n_inst;
     struct Quiet {
         bool ok = false;
@@ -791,6 +798,10 @@ bool ensure_batch_loop(Batch* b) {
     return true;
 }
 
+int64_t batch_loop_shortest(const Batch* b, int64_t max_iter) {
+    return loop_shortest(b->loop.form, b->loop.faces, b->loop.threads, b->loop.sectors, true, max_iter);
+}
+
 // One launch of the batched loop for `iters` iterations of every active
 // instance (h_inst is up to date); false also when one of its waits gave up,
 // and, with no error set, when the launch was refused (its blocks do not fit
@@ -822,7 +833,7 @@ bool launch_loop(Batch* b, float cfl, double tol, int iters, cudaStream_t s, boo
                              s), what))
         return false;
     const cudaError_t e = L.refuse ? cudaErrorCooperativeLaunchTooLarge
-                                   : launch_batch_loop(L.d_inst, L.d_inst_of_block, L.blocks, L.faces, L.threads,
+                                   : launch_batch_loop(L.d_inst, L.d_inst_of_block, L.blocks, L.form, L.faces, L.threads,
                                                        reference_momentum(), s);
     L.refuse = false;
     if (e != cudaSuccess) {
@@ -881,15 +892,13 @@ int64_t run_loop(Batch* b, float cfl, int64_t max_iter, double tol, int check_ev
     };
     const bool persistent = b->variant >= kPersistentVariant;
     // The batched loop in place of the default form's kernels (with its tile
-    // the residual's sums are the same too), where the instances fit and a
-    // launch pays for loading the geometry.  Measured per iteration against
-    // the graph, us (B200): 100 iterations of 2 x 4,608 prisms 11.4 / 21.0, 10
-    // instances of 57,168 together 15.7 / 23.1, 1 x 50,000 12.7 / 23.0, 1 x
-    // 120,000 18.6 / 36.6; 4 iterations a launch 29.5 / 35.6, 33.9 / 37.4, 30.1 /
-    // 37.2, and 9 of the 120,000 30.5 / 40.3.
+    // the residual's sums are the same too), where the instances fit, its form
+    // is the faster one and a launch pays for loading the geometry
+    // (loop_shape.h).  Per iteration against the graph, us (B200): 10 instances
+    // of 57,168 prisms together 15.7 / 23.1.
     const int64_t chunk0 = std::min<int64_t>(check_every, max_iter);
     bool loop = b->variant == 0 && b->tile == kBlock && chunk0 >= 4 && ensure_batch_loop(b) &&
-                chunk0 >= (b->loop.threads <= kLoopWide ? 4 : 8);
+                chunk0 >= batch_loop_shortest(b, max_iter);
     ok = ok && (loop || (build_items(b) && (persistent || capture())));
     const int tuned = b->tile;
     int64_t done = 0;
@@ -1186,7 +1195,10 @@ int gbBatchAutotune(gbBatch* b, gb_scalar cfl, int trial_iters, int* tile_out, i
                 bool refused = false;
                 b->table_stale = true;
                 ok = launch_loop(b, cfl, 0.0, 4, s, &refused);
-                if (refused) ok = !(loop = false);
+                if (refused) {
+                    loop = false;
+                    ok = true;
+                }
                 ok = ok && download_inst(b);
             }
             if (ok && !loop) enqueue_iteration(b, cfl, 0.0, s);

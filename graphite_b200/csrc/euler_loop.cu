@@ -422,7 +422,7 @@ __device__ __forceinline__ void euler_loop_worker(const EulerLoopArgs& a, const 
     }
 }
 
-template <bool TRANSPOSED, int MAXF, int THREADS, bool LEAN>
+template <bool TRANSPOSED, int MAXF, int THREADS, LoopForm FORM>
 __global__ void __launch_bounds__(THREADS, kLoopBlocksPerSM) k_euler_loop(const __grid_constant__ EulerLoopArgs a) {
     extern __shared__ float s_geo[];
     __shared__ GhostBcTable s_bc;
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(THREADS, kLoopBlocksPerSM) k_euler_loop(const 
     for (unsigned int k = threadIdx.x; k < sizeof(GhostBcTable) / 4; k += blockDim.x)
         reinterpret_cast<uint32_t*>(&s_bc)[k] = reinterpret_cast<const uint32_t*>(&a.ghosts)[k];
     __syncthreads();
-    euler_loop_worker<TRANSPOSED, MAXF, (THREADS <= kLoopWide), LEAN>(a, s_bc, blockIdx.x, s_geo);
+    euler_loop_worker<TRANSPOSED, MAXF, FORM == LoopForm::kWide, FORM == LoopForm::kLean>(a, s_bc, blockIdx.x, s_geo);
 }
 
 // k_batch_reduce for one instance of the batched loop.
@@ -474,7 +474,7 @@ __device__ void batch_reducer(const BatchLoopInst& a) {
 // and nothing waits across instances.  Per iteration against the replayed
 // graph of three kernels (B200): 2 instances of 4,608 prisms 11.4 / 21.0 us, 10
 // of 57,168 together 15.7 / 23.1, 40 of 92,160 together 20.0 / 33.2.
-template <bool TRANSPOSED, int MAXF, int THREADS>
+template <bool TRANSPOSED, int MAXF, int THREADS, LoopForm FORM>
 __global__ void __launch_bounds__(THREADS, kLoopBlocksPerSM)
     k_euler_loop_batch(const BatchLoopInst* __restrict__ insts, const int* __restrict__ inst_of_block) {
     extern __shared__ float s_geo[];
@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(THREADS, kLoopBlocksPerSM)
     if (a.iters == 0) return;                     // stopped before
     const uint32_t block = blockIdx.x - (uint32_t)a.first_block;
     if (block == (uint32_t)a.n_blocks) batch_reducer(a);
-    else euler_loop_worker<TRANSPOSED, MAXF, (THREADS <= kLoopWide), false>(a, a.ghosts, block, s_geo);
+    else euler_loop_worker<TRANSPOSED, MAXF, FORM == LoopForm::kWide, false>(a, a.ghosts, block, s_geo);
 }
 
 // off[g]: ghost g's face centre - its centroid
@@ -498,13 +498,12 @@ __global__ void k_ghost_off(MeshDev m, uint32_t G, const uint2* __restrict__ gho
 }
 
 template <bool TRANSPOSED, int MAXF>
-cudaError_t launch(EulerLoopArgs& a, int threads, cudaStream_t s) {
-    const bool lean = loop_lean(MAXF, threads);
-    const void* fn = lean                   ? (const void*)k_euler_loop<TRANSPOSED, MAXF, kLoopMax, true>
-                     : threads <= kLoopWide ? (const void*)k_euler_loop<TRANSPOSED, MAXF, kLoopWide, false>
-                     : threads <= 320       ? (const void*)k_euler_loop<TRANSPOSED, MAXF, 320, false>
-                                            : (const void*)k_euler_loop<TRANSPOSED, MAXF, kLoopFull, false>;
-    const int smem = loop_smem(MAXF, threads);
+cudaError_t launch(EulerLoopArgs& a, LoopForm form, int threads, cudaStream_t s) {
+    const void* fn = form == LoopForm::kWide   ? (const void*)k_euler_loop<TRANSPOSED, MAXF, kLoopWide, LoopForm::kWide>
+                     : form == LoopForm::kLean ? (const void*)k_euler_loop<TRANSPOSED, MAXF, kLoopMax, LoopForm::kLean>
+                     : threads <= 320          ? (const void*)k_euler_loop<TRANSPOSED, MAXF, 320, LoopForm::kNarrow>
+                                      : (const void*)k_euler_loop<TRANSPOSED, MAXF, kLoopFull, LoopForm::kNarrow>;
+    const int smem = loop_smem(form, MAXF, threads);
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     void* args[] = {(void*)&a};
@@ -514,10 +513,12 @@ cudaError_t launch(EulerLoopArgs& a, int threads, cudaStream_t s) {
 }
 
 template <bool TRANSPOSED, int MAXF>
-cudaError_t launch_batch(const BatchLoopInst* insts, const int* inst_of_block, int blocks, int threads, cudaStream_t s) {
-    const void* fn = threads <= kLoopWide ? (const void*)k_euler_loop_batch<TRANSPOSED, MAXF, kLoopWide>
-                                          : (const void*)k_euler_loop_batch<TRANSPOSED, MAXF, kLoopFull>;
-    const int smem = loop_smem(MAXF, threads);
+cudaError_t launch_batch(const BatchLoopInst* insts, const int* inst_of_block, int blocks, LoopForm form, int threads,
+                         cudaStream_t s) {
+    const void* fn = form == LoopForm::kWide
+                         ? (const void*)k_euler_loop_batch<TRANSPOSED, MAXF, kLoopWide, LoopForm::kWide>
+                         : (const void*)k_euler_loop_batch<TRANSPOSED, MAXF, kLoopFull, LoopForm::kNarrow>;
+    const int smem = loop_smem(form, MAXF, threads);
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     void* args[] = {(void*)&insts, (void*)&inst_of_block};
@@ -528,13 +529,13 @@ cudaError_t launch_batch(const BatchLoopInst* insts, const int* inst_of_block, i
 
 }  // namespace
 
-cudaError_t launch_batch_loop(const BatchLoopInst* insts, const int* inst_of_block, int blocks, int max_faces,
-                              int threads, bool transposed, cudaStream_t s) {
+cudaError_t launch_batch_loop(const BatchLoopInst* insts, const int* inst_of_block, int blocks, LoopForm form,
+                              int max_faces, int threads, bool transposed, cudaStream_t s) {
     auto go = [&](auto tr) {
         constexpr bool T = decltype(tr)::value;
-        if (max_faces <= 4) return launch_batch<T, 4>(insts, inst_of_block, blocks, threads, s);
-        if (max_faces == 5) return launch_batch<T, 5>(insts, inst_of_block, blocks, threads, s);
-        return launch_batch<T, 6>(insts, inst_of_block, blocks, threads, s);
+        if (max_faces <= 4) return launch_batch<T, 4>(insts, inst_of_block, blocks, form, threads, s);
+        if (max_faces == 5) return launch_batch<T, 5>(insts, inst_of_block, blocks, form, threads, s);
+        return launch_batch<T, 6>(insts, inst_of_block, blocks, form, threads, s);
     };
     return transposed ? go(std::true_type{}) : go(std::false_type{});
 }
@@ -545,10 +546,11 @@ void launch_ghost_off(const DevMesh& d, float4* ghost_off, cudaStream_t s) {
     count_launch();
 }
 
-cudaError_t launch_euler_loop(EulerLoopArgs& a, int max_faces, int threads, bool transposed, cudaStream_t s) {
-    if (max_faces <= 4) return transposed ? launch<true, 4>(a, threads, s) : launch<false, 4>(a, threads, s);
-    if (max_faces == 5) return transposed ? launch<true, 5>(a, threads, s) : launch<false, 5>(a, threads, s);
-    return transposed ? launch<true, 6>(a, threads, s) : launch<false, 6>(a, threads, s);
+cudaError_t launch_euler_loop(EulerLoopArgs& a, LoopForm form, int max_faces, int threads, bool transposed,
+                              cudaStream_t s) {
+    if (max_faces <= 4) return transposed ? launch<true, 4>(a, form, threads, s) : launch<false, 4>(a, form, threads, s);
+    if (max_faces == 5) return transposed ? launch<true, 5>(a, form, threads, s) : launch<false, 5>(a, form, threads, s);
+    return transposed ? launch<true, 6>(a, form, threads, s) : launch<false, 6>(a, form, threads, s);
 }
 
 }  // namespace gb

@@ -5,11 +5,6 @@
 
 namespace gb {
 
-// One cell per thread.  Up to kLoopWide threads per block a thread may use
-// 128 registers and keeps its own face states and ghosts in shared memory.
-constexpr int kLoopWide = 256;
-constexpr int kLoopFull = 416;          // all of a cell's geometry in shared memory up to here
-constexpr int kLoopMax = 512;
 struct EulerLoopArgs : LoopArgs {
     MeshDev m;
     const float4* ghost_off;              // per ghost: its face centre - its centroid
@@ -25,17 +20,6 @@ struct EulerLoopArgs : LoopArgs {
     TagRec* rec;                          // 2 per entry: (rho, u, v), (w, E)
 };
 
-// shared memory of a block (bytes); lean: without the face normals and areas
-constexpr int loop_smem_of(int max_faces, int threads, bool lean) {
-    return threads * ((lean ? 28 : 44) * max_faces + 28 + (threads <= kLoopWide && !lean ? 64 + 28 * max_faces : 0));
-}
-constexpr bool loop_lean(int max_faces, int threads) {
-    return threads > kLoopFull || loop_smem_of(max_faces, threads, false) > kLoopSmem;
-}
-constexpr int loop_smem(int max_faces, int threads) {
-    return loop_smem_of(max_faces, threads, loop_lean(max_faces, threads));
-}
-
 // One instance of a batch in the batched loop: its own workers and reducer,
 // and what k_batch_reduce keeps of it.
 struct BatchLoopInst : EulerLoopArgs {
@@ -47,10 +31,12 @@ struct BatchLoopInst : EulerLoopArgs {
 };
 
 void launch_ghost_off(const DevMesh& d, float4* ghost_off, cudaStream_t s);
-cudaError_t launch_euler_loop(EulerLoopArgs& a, int max_faces, int threads, bool transposed, cudaStream_t s);
-// blocks: of the grid; inst_of_block: the instance of each.  threads <= kLoopFull.
-cudaError_t launch_batch_loop(const BatchLoopInst* insts, const int* inst_of_block, int blocks, int max_faces,
-                              int threads, bool transposed, cudaStream_t s);
+// form: loop_form(max_faces, threads)
+cudaError_t launch_euler_loop(EulerLoopArgs& a, LoopForm form, int max_faces, int threads, bool transposed,
+                              cudaStream_t s);
+// blocks: of the grid; inst_of_block: the instance of each.  WIDE or NARROW.
+cudaError_t launch_batch_loop(const BatchLoopInst* insts, const int* inst_of_block, int blocks, LoopForm form,
+                              int max_faces, int threads, bool transposed, cudaStream_t s);
 
 MeshDev mesh_dev(const DevMesh& m);
 

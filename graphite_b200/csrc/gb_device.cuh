@@ -256,6 +256,8 @@ struct MeshAccess {
     Workspace* ws;
 };
 bool mesh_access(::cuMesh* mesh, MeshAccess* out);
+// neighbour_sectors of the mesh, counted at its first use
+float mesh_sectors(::cuMesh* mesh);
 bool reference_momentum();
 
 // Device buffers of a field (device cell order; val[cur] is the current value).

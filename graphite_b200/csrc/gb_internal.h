@@ -65,4 +65,9 @@ struct Numbering {
 
 void number_cells(const Topology& t, bool rcm, Numbering& num);
 
+// 32-byte sectors that the 32 lanes of a warp (consecutive interior cells) touch
+// when they read their neighbours' 16-byte records, all face slots together:
+// the mean over up to 128 warps.
+float neighbour_sectors(const Numbering& num);
+
 }  // namespace gb

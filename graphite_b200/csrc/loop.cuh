@@ -4,6 +4,7 @@
 #pragma once
 
 #include "euler_ops.cuh"
+#include "loop_shape.h"
 
 namespace gb {
 
@@ -15,7 +16,6 @@ struct alignas(16) TagRec {
 
 // One cell per thread, two blocks per SM.
 constexpr int kLoopBlocksPerSM = 2;
-constexpr int kLoopSmem = 112 * 1024;   // dynamic shared memory of a block, at most
 // Polls of a wait before it gives up (a poll takes about half a microsecond).
 constexpr unsigned int kLoopSpinLimit = 1u << 23;
 

@@ -669,6 +669,29 @@ bool read_fvm(const char* path, Topology& t) {
     return true;
 }
 
+float neighbour_sectors(const Numbering& num) {
+    const int64_t N = (int64_t)num.start.size() - 1, warps = (N + 31) / 32, sampled = std::min<int64_t>(warps, 128);
+    int64_t sectors = 0;
+    for (int64_t k = 0; k < sampled; ++k) {
+        const int64_t i0 = 32 * (k * warps / sampled), i1 = std::min(N, i0 + 32);
+        for (uint32_t t = 0;; ++t) {                 // face slot
+            uint32_t s[32];
+            int n = 0;
+            bool more = false;
+            for (int64_t i = i0; i < i1; ++i) {
+                if (t >= num.start[i + 1] - num.start[i]) continue;
+                more = true;
+                const uint32_t j = num.nb_cell[num.start[i] + t];
+                if (j < (uint64_t)N) s[n++] = j / 2;
+            }
+            if (!more) break;
+            std::sort(s, s + n);
+            sectors += std::unique(s, s + n) - s;
+        }
+    }
+    return sampled ? (float)sectors / (float)sampled : 0.f;
+}
+
 // Reverse Cuthill-McKee over the interior-cell graph, ghosts by region,
 // faces by (lower, higher) new cell index.
 void number_cells(const Topology& t, bool rcm, Numbering& num) {

@@ -272,8 +272,9 @@ int gbApplyBoundaryConditions(cuMesh* mesh);
 
 /* Runs n_iter iterations of the PhysicsEuler::step loop (boundary conditions
  * in the given order, prepare, step, residual sum) as a replayed CUDA graph,
- * or, on meshes that fit on the GPU one cell per thread (about 150,000 cells),
- * as one persistent cooperative launch per check_every iterations,
+ * or, on meshes that fit on the GPU one cell per thread (about 150,000 cells)
+ * and where that is the faster form, as one persistent cooperative launch per
+ * check_every iterations,
  * writing the residual sum of each iteration to residual_history (host
  * array of n_iter doubles, may be NULL).  With tolerance > 0 it stops after
  * the first iteration in which residual/residual[0] < tolerance: the device
@@ -353,7 +354,8 @@ int gbBatchGetState(gbBatch* batch, int instance, float* rho, float* rhou, float
  * compiles the gradient and flux kernels for 4 / 5 resident 256-thread blocks
  * per SM (variant 0 stages the entries as variant 2 does from 300,000 active
  * cells, and with 256-cell tiles runs as one persistent launch per check_every
- * iterations where the instances fit on the GPU one cell per thread), variant 2
+ * iterations where the instances fit on the GPU one cell per thread and that
+ * is the faster form), variant 2
  * runs the gradient pass in 128-thread blocks that stage
  * each cell's face entries in shared memory (flux as variant 1), variants 3
  * and 4 are one persistent cooperative kernel per check_every iterations
