@@ -6,9 +6,9 @@
 // forbid other allocations, and plugins that must keep their device footprint
 // fixed after setup.  The mesh/field entry points allocate their
 // scratch (reduction partials, gradients) on first use; this entry point
-// allocates nothing.  Its scratch -- one float64 partial sum per block of
-// 2048 inputs -- lives in the file-scope array below, which every GPU that
-// loads the library holds until the process exits.
+// allocates nothing.  Its scratch -- a float64 partial sum per block and the
+// calls' arrival counters -- lives in the file-scope array below, which every
+// GPU that loads the library holds until the process exits.
 #include <algorithm>
 #include <atomic>
 #include <mutex>
@@ -26,14 +26,17 @@ constexpr int64_t kNoAllocBlockItems = (int64_t)kBlock * 8;      // inputs per b
 constexpr int64_t kNoAllocMaxItems = (int64_t)kNoAllocPartials * kNoAllocBlockItems;   // 8,388,608
 constexpr int kMaxDevices = 64;
 
-// Arrival counters of the calls, taken in turn, after the partial sums: calls
-// that overlap race for the partial sums, but not for one counter, so every
-// counter is back at zero when its call has ended.
+// Arrival counters of the calls, taken in turn, after the partial sums.  What
+// the blocks of a call add to its counter comes to zero (modulo 2^32), so a
+// counter is at zero again once every call that used it has ended, even if
+// calls overlapped on it (more than 64 in flight, or a captured call, which
+// keeps its counter, replayed beside another): an overlap can spoil the
+// results of the calls that overlap, never those of later ones.
 constexpr int kCounters = 64;
 static __device__ __align__(256) double g_noalloc_partials[kNoAllocPartials + kCounters];
 
 constexpr int kSumThreads = 512;
-constexpr int kSumMaxBlocks = 592;        // four per SM: 2.4 M values in flight hide the memory's latency
+constexpr int kSumMaxBlocks = 592;        // 444 resident at once (34 registers, three per SM), then the rest
 
 __device__ __forceinline__ double sum_block(double x) {
     __shared__ double w[kSumThreads / 32];
@@ -84,13 +87,14 @@ __global__ void __launch_bounds__(kSumThreads) k_sum(int64_t n, const float* __r
         return;
     }
     if (threadIdx.x == 0) {
+        // block 0 adds 1 - gridDim.x, the others 1: zero only when all have arrived
+        const unsigned int add = blockIdx.x == 0 ? 1u - gridDim.x : 1u;
         partials[blockIdx.x] = bs;
         __threadfence();
-        last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+        last = atomicAdd(arrived, add) + add == 0u;
     }
     __syncthreads();
     if (!last) return;
-    if (threadIdx.x == 0) *arrived = 0;
     __threadfence();
     double s = 0.0;
     for (int k = threadIdx.x; k < (int)gridDim.x; k += kSumThreads) s += __ldcg(&partials[k]);

@@ -600,8 +600,9 @@ int gbNSIWallForce(cuMesh* mesh, FvmField* velocity, FvmField* pressure, unsigne
  * device looks the array's address up (cudaGetSymbolAddress) and keeps it;
  * that address does not survive a cudaDeviceReset of that device.  All
  * calls share the array: calls that
- * overlap on the GPU (other streams, other threads) race and must be ordered
- * by the caller.  Asynchronous on `stream` (a cudaStream_t; NULL = legacy
+ * overlap on the GPU (other streams, other threads, replays of a captured
+ * call) race and must be ordered by the caller; an overlap can spoil the
+ * results of the calls that overlap, not those of later ones.  Asynchronous on `stream` (a cudaStream_t; NULL = legacy
  * default stream).  Returns 0, or nonzero with gbGetLastError set.  No
  * counterpart in the reference. */
 int gbReduceSumNoAlloc(const float* values, uint64_t n, double* result, void* stream);
