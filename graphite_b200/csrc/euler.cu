@@ -309,17 +309,18 @@ __global__ void k_scatter_vector(int64_t n, const float* __restrict__ src, const
     if (i < n) dst[idx[i]] = make_float4(src[3 * i], src[3 * i + 1], src[3 * i + 2], 0.f);
 }
 
-// one thread per value component: consecutive threads write consecutive triples
-__global__ void k_gather_gradients(int64_t n, uint32_t N, int comps, const float4* __restrict__ grad,
+// one thread per value component of [k0, k0 + m): consecutive threads write consecutive triples
+__global__ void k_gather_gradients(int64_t k0, int64_t m, uint32_t N, int comps, const float4* __restrict__ grad,
                                    const uint32_t* __restrict__ cell_new, const uint2* __restrict__ ghost, float* g,
                                    float* l) {
-    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n * comps) return;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= m) return;
+    const int64_t k = k0 + t;
     uint32_t i = cell_new[k / comps];
     if (i >= N) i = ghost[i - N].x;
     const float4 v = grad[(size_t)i * comps + k % comps];
-    g[3 * k] = v.x; g[3 * k + 1] = v.y; g[3 * k + 2] = v.z;
-    l[k] = v.w;
+    g[3 * t] = v.x; g[3 * t + 1] = v.y; g[3 * t + 2] = v.z;
+    l[t] = v.w;
 }
 
 __global__ void k_gather_state(int64_t n, const float* __restrict__ rho, const float4* __restrict__ rhou,
@@ -468,11 +469,10 @@ void launch_scatter_vector(int64_t n, const float* src3, const uint32_t* idx, fl
     count_launch();
 }
 
-void launch_gather_gradients(const DevMesh& m, int comps, const float4* grad, const uint32_t* cell_new, float* g,
-                             float* l, cudaStream_t s) {
-    const int64_t n = m.N + m.G;
+void launch_gather_gradients(const DevMesh& m, int comps, const float4* grad, const uint32_t* cell_new, int64_t k0,
+                             int64_t n, float* g, float* l, cudaStream_t s) {
     if (n == 0) return;
-    k_gather_gradients<<<grid(n * comps), kBlock, 0, s>>>(n, (uint32_t)m.N, comps, grad, cell_new, m.ghost, g, l);
+    k_gather_gradients<<<grid(n), kBlock, 0, s>>>(k0, n, (uint32_t)m.N, comps, grad, cell_new, m.ghost, g, l);
     count_launch();
 }
 

@@ -213,10 +213,10 @@ void launch_gather_scalar(int64_t n, const float* src, const uint32_t* idx, floa
 void launch_gather_vector(int64_t n, const float4* src, const uint32_t* idx, float* dst3, cudaStream_t s);
 void launch_scatter_scalar(int64_t n, const float* src, const uint32_t* idx, float* dst, cudaStream_t s);
 void launch_scatter_vector(int64_t n, const float* src3, const uint32_t* idx, float4* dst, cudaStream_t s);
-// a field's gradients + limiters (cell order of the mesh) in the host mirrors' layout and order: g[n][comps][3] and
-// l[n][comps] for n cells and ghosts, a ghost carrying its interior cell's
-void launch_gather_gradients(const DevMesh& m, int comps, const float4* grad, const uint32_t* cell_new, float* g,
-                             float* l, cudaStream_t s);
+// a field's gradients + limiters (cell order of the mesh) in the host mirrors' layout and order, g[][comps][3] and
+// l[][comps] over cells and ghosts, a ghost carrying its interior cell's: the n value components from the k0-th on
+void launch_gather_gradients(const DevMesh& m, int comps, const float4* grad, const uint32_t* cell_new, int64_t k0,
+                             int64_t n, float* g, float* l, cudaStream_t s);
 // a whole state between device order and stage = rho[n], rhou[3n], rhoe[n] in reference order; scatter writes both
 // value buffers
 void launch_gather_state(int64_t n, const float* rho, const float4* rhou, const float* rhoe, const uint32_t* idx,
