@@ -1189,7 +1189,9 @@ int gbBatchAutotune(gbBatch* b, gb_scalar cfl, int trial_iters, int* tile_out, i
             b->variant = c.variant;
             reset_counters(b, 1 << 30, false);
             ok = ok && size_partials(b) && build_items(b) && upload_inst(b);
-            // one untimed iteration (or launch of the loop, where a run would take it), then the timed trial
+            // one untimed iteration (or launch of the loop, which a run takes in place of these kernels where it fits;
+            // trials of fewer than 4 iterations time the kernels, which rank it among the first on such batches
+            // already), then the timed trial
             bool loop = ok && c.variant == 0 && c.tile == kBlock && iters >= 4 && ensure_batch_loop(b);
             if (loop) {
                 bool refused = false;
