@@ -1705,6 +1705,7 @@ int gbFieldInit(cuMesh* mesh, FvmField* u, gb_vector value) {
     if (!check_mesh(mesh)) return 1;
     FieldImpl* fi = impl(u);
     if (!fi || !bind(mesh, u, fi->comps, "gbFieldInit") || !flush_for(u)) return 1;
+    fi->partials_valid = false;          // of an error field that a step has summed
     const int64_t n_grad = fi->grad ? impl(mesh)->dev.N * fi->comps : 0;
     launch_field_init((int64_t)fi->size, fi->comps, fi->val[0], fi->val[1], make_float4(value.x, value.y, value.z, 0.f),
                       n_grad, fi->grad, t_stream);
@@ -1769,6 +1770,7 @@ int gbFieldAxpy(cuMesh* mesh, FvmField* y, gb_scalar a, FvmField* x) {
     if (!bind(mesh, y, fy->comps, "gbFieldAxpy") || !bind(mesh, x, fy->comps, "gbFieldAxpy") || !flush_for(x) ||
         !flush_for(y))
         return 1;
+    fy->partials_valid = false;
     launch_field_axpy(impl(mesh)->dev, fy->comps, a, fx->val[fx->cur], fy->val[fy->cur], t_stream);
     return launch_ok("gbFieldAxpy") ? 0 : 1;
 }
@@ -1831,6 +1833,7 @@ int gbFvmApplyTerms(cuMesh* mesh, int n_terms, const gbFvmTerm* terms, FvmField*
     if (!out) { set_error("gbFvmApplyTerms: null output field"); return 1; }
     if (!bind(mesh, out, oc, what) || !flush_for(out)) return 1;
     FieldImpl* fo = impl(out);
+    fo->partials_valid = false;
     launch_fvm_terms(impl(mesh)->dev, oc, n_terms, dt, oc == 1 ? (float*)fo->val[fo->cur] : nullptr,
                      oc == 3 ? (float4*)fo->val[fo->cur] : nullptr, t_stream);
     return launch_ok(what) ? 0 : 1;
