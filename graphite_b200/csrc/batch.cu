@@ -720,14 +720,18 @@ bool ensure_batch_loop(Batch* b) {
     if (L.form != LoopForm::kWide && L.form != LoopForm::kNarrow) return false;
     if (loop_shortest(L.form, L.faces, threads, L.sectors, true, 0) == kLoopNever) return false;
     L.blocks = (int)blocks_at(threads) + b->n_inst;
+    // where there is no memory for all of it, none of it is kept
     struct Quiet {
+        std::vector<void*>& allocations;
+        const size_t before = allocations.size();
         bool ok = false;
         ~Quiet() {
             if (ok) return;
+            for (; allocations.size() > before; allocations.pop_back()) cudaFree(allocations.back());
             clear_error();
             cudaGetLastError();
         }
-    } quiet;
+    } quiet{b->allocations};
     cudaStream_t s = (cudaStream_t)gbGetStream();
     std::vector<float4*> off(b->meshes.size(), nullptr);
     const char* what = "batch loop";
