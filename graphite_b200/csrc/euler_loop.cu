@@ -18,16 +18,20 @@
 // (go on, converged, not finite) is waited for by the update of the next
 // iteration, behind that iteration's gradient pass.
 //
-// What bounds it: up to about 400 cells per SM the latency of one cell's
-// chain -- two hand-overs through L2 of about 1 us each and the dependent
-// arithmetic of a gradient and a flux -- so a thread gathers all its
-// neighbours at once and keeps what it can on chip; beyond that the issue
-// slots, so a thread takes its faces one at a time in few registers.  Measured
-// per iteration against the replayed graph of four kernels (B200): 4,608
-// prisms 10.1 / 17.7 us, 28,800 tets 11.0 / 20.3, 50,000 prisms 12.1 / 21.9,
-// 120,000 prisms 16.8 / 27.5, 140,736 prisms (normals read from L2) 29.1 / 30.0.
-// With a state's two records side by side instead of in planes the 120,000
-// prisms took 19.5.
+// What bounds it is latency: a cell's chain in an iteration is two hand-overs
+// through L2 of about 1 us each and the dependent arithmetic of a gradient and
+// a flux, and one cell per thread leaves few warps to hide it.  Counters (B200):
+// 28,800 tets, 6 warps per SM, issue slots 21 % busy, L2 at 10 % of its
+// throughput, 3.2 warps waiting for memory per instruction issued; 120,000
+// prisms, 25 warps, 47 %, 36 %, 8.3.  So the wide form gathers all of a cell's
+// neighbours at once and keeps what it can on chip; the narrow ones have one
+// face in flight in few registers and live off their warps.  Per iteration in
+// launches of 100 against the replayed graph of three or four kernels: 12,060
+// prisms in one layer 11.3 / 19.1 us, 28,350 tets 10.5 / 19.1, 45,240 prisms 13.0 /
+// 21.1, 74,148 prisms 13.2 / 23.1, 120,416 prisms 18.8 / 27.2, 148,208 prisms
+// (normals read from L2) 21.8 / 33.4; where it loses and is not taken:
+// loop_shape.h.  With a state's two records side by side instead of in planes
+// 120,000 prisms took 19.5 where they took 16.8.
 // Flags per block instead of tagged data took 12 to 21 us for these: a fence
 // on each side and a block barrier per hand-over, and the slowest warp of
 // every block in everyone's way.
@@ -90,9 +94,8 @@ struct TileGeo {
     __device__ __forceinline__ float3 cf3(int t) const { return f3(cf4(t)); }
 };
 
-// The neighbour word: the neighbour's cell index and, in the top four bits,
-// the slot of the same face among its entries, or a ghost's region.
-constexpr uint32_t kNbMask = (1u << 28) - 1u;
+// In the top four bits of the neighbour word (kNbMask): the slot of the same
+// face among the neighbour's entries, or a ghost's region.
 
 template <int MAXF, bool WIDE, bool LEAN>
 __device__ __forceinline__ void load_geo(const EulerLoopArgs& a, uint32_t i, int nf, const TileGeo<MAXF, LEAN>& g) {
@@ -497,6 +500,9 @@ __global__ void k_ghost_off(MeshDev m, uint32_t G, const uint2* __restrict__ gho
     off[g] = make_float4(d.x, d.y, d.z, 0.f);
 }
 
+// Two blocks per SM leave a thread 96 registers up to 320 threads per block and
+// 72 up to 416: with 72 for all, 78,000 prisms took 16.5 us per iteration (14.9
+// with 96) and 90,000 15.9 (14.6).
 template <bool TRANSPOSED, int MAXF>
 cudaError_t launch(EulerLoopArgs& a, LoopForm form, int threads, cudaStream_t s) {
     const void* fn = form == LoopForm::kWide   ? (const void*)k_euler_loop<TRANSPOSED, MAXF, kLoopWide, LoopForm::kWide>

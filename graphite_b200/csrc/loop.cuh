@@ -24,6 +24,9 @@ constexpr unsigned int loop_spin_start(unsigned int polls) {
     return polls == 0 || polls > kLoopSpinLimit ? 0u : kLoopSpinLimit - polls;
 }
 
+// A cell's neighbour word: the neighbour's index below its top four bits.
+constexpr uint32_t kNbMask = (1u << 28) - 1u;
+
 struct LoopArgs {
     uint32_t N;
     int iters, cur0;                      // iterations of the launch, value buffer it starts from

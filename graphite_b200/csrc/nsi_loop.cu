@@ -7,11 +7,14 @@
 // the viscous flux needs the whole velocity gradient.  A new state is written
 // after reading the neighbours' gradients, which they form after reading the
 // old one; new gradients after reading the neighbours' new states, which they
-// form after reading the old gradients.  Bound like euler_loop.cu: by the
-// latency of a cell's chain up to about 400 cells per SM, then by what the
-// fluxes read from L2 (96 bytes per face).  Per iteration against the replayed
-// graph of three kernels (B200): 1,152 hexes 7.4 / 19.9 us, 28,800 tets 8.3 /
-// 26.6, 60,000 hexes 10.4 / 24.1, 100,000 hexes 20.1 / 29.1.
+// form after reading the old gradients.  Bound like euler_loop.cu by the latency
+// of a cell's chain: 100,000 hexes in one layer, 21 warps per SM, issue slots
+// 39 % busy, L2 at 16 % of its throughput, 7.9 warps waiting for memory per
+// instruction issued.  Per iteration in launches of 100 against the replayed
+// graph (B200): 27,984 hexes in one layer 7.9 / 19.9 us, 28,350 tets 7.5 / 27.2,
+// 54,096 hexes 8.9 / 22.9, 89,823 hexes 20.3 / 27.4, 104,960 hexes 22.4 / 29.1; with
+// the limiter 14.4 / 24.2, 16.2 / 33.3, 15.4 / 26.3, 27.6 / 30.7 and 29.1 / 31.3; where
+// it loses and is not taken: loop_shape.h.
 #include "nsi_loop.cuh"
 
 #include <algorithm>
@@ -24,7 +27,6 @@ namespace {
 // offsets of the neighbour, of the face centre and of the face centre from the
 // neighbour, with WIDE the outward normal and area / volume; then the
 // least-squares inverse and the volume.
-constexpr uint32_t kNbMask = (1u << 28) - 1u;
 template <int MAXF, bool WIDE>
 struct NsiGeo {
     static constexpr int kLsq = (WIDE ? 14 : 10) * MAXF;
@@ -309,6 +311,10 @@ __global__ void __launch_bounds__(THREADS, kLoopBlocksPerSM) k_nsi_loop(const __
     }
 }
 
+// Registers a thread: 128, 80 up to 352 threads per block, 72 up to 448, 64.  With
+// 64 for all above 256 threads 90,000 hexes took 24.6 us per iteration (18.4), 112,000
+// 30.0 (20.7), 126,000 tets 31.8 (21.6), with the limiter 31.9 (26.7), 36.6 (29.9) and
+// 45.7 (39.3).
 template <int MAXF>
 cudaError_t launch(NsiLoopArgs& a, int threads, cudaStream_t s) {
     const void* fn = threads <= kNsiWide ? (const void*)k_nsi_loop<MAXF, kNsiWide>
