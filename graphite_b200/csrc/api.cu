@@ -164,6 +164,12 @@ struct FieldImpl {
     // before anything reads or writes the field
     FieldBcTable bcs{};
     bool bcs_pending = false;
+    // What a caller ordered against the calls that asked for them stays ordered
+    // against the launch: from_event is recorded when the first one is asked
+    // for, done_event behind the launch on done_stream (valid: done)
+    cudaEvent_t from_event = nullptr, done_event = nullptr;
+    cudaStream_t done_stream = nullptr;
+    bool done = false;
 };
 
 MeshImpl* impl(cuMesh* m) { return m ? static_cast<MeshImpl*>(m->impl) : nullptr; }
@@ -361,13 +367,53 @@ bool check_mesh(cuMesh* m) {
     return true;
 }
 
-// Applies the field's pending conditions, if any.
+// Whether the thread's stream is being captured into a graph by its owner.
+bool capturing() {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(t_stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return false;
+}
+
+// Lets a thread whose stream is being captured work on another stream.
+struct OutsideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Applies the field's pending conditions, if any, and orders the thread's
+// stream behind the last application: it may have been launched on another
+// stream, later than the call that asked for it.
 bool flush_field_bcs(cuMesh* mesh, FvmField* f) {
+    const char* what = "field boundary conditions";
     FieldImpl* fi = impl(f);
+    if (!fi->bcs_pending && (!fi->done || fi->done_stream == t_stream)) return true;
+    const bool captured = capturing();
+    if (fi->done && fi->done_stream != t_stream) {
+        if (captured) {
+            OutsideCapture oc;
+            if (!cuda_ok(cudaEventSynchronize(fi->done_event), what)) return false;
+            fi->done = false;
+        } else if (!cuda_ok(cudaStreamWaitEvent(t_stream, fi->done_event, 0), what)) {
+            return false;
+        }
+    }
     if (!fi->bcs_pending) return true;
     fi->bcs_pending = false;
-    launch_field_bc(impl(mesh)->dev, fi->comps, fi->bcs, fi->cur, fi->val[0], fi->val[1], t_stream);
-    return launch_ok("field boundary conditions");
+    MeshImpl* mi = impl(mesh);
+    if (captured) {
+        // asked for before the capture: no part of the graph, and done before it can be launched
+        OutsideCapture oc;
+        if (!mi->capture && !cuda_ok(cudaStreamCreateWithFlags(&mi->capture, cudaStreamNonBlocking), what)) return false;
+        if (!cuda_ok(cudaStreamWaitEvent(mi->capture, fi->from_event, 0), what)) return false;
+        launch_field_bc(mi->dev, fi->comps, fi->bcs, fi->cur, fi->val[0], fi->val[1], mi->capture);
+        return launch_ok(what) && cuda_ok(cudaStreamSynchronize(mi->capture), what);
+    }
+    launch_field_bc(mi->dev, fi->comps, fi->bcs, fi->cur, fi->val[0], fi->val[1], t_stream);
+    fi->done_stream = t_stream;
+    fi->done = true;
+    return launch_ok(what) && cuda_ok(cudaEventRecord(fi->done_event, t_stream), what);
 }
 
 // Binds a field's device storage to a mesh's cell order (first use).  Every
@@ -1034,7 +1080,10 @@ void FvmFieldFree(FvmField* f) {
     if (!f) return;
     FieldImpl* fi = impl(f);
     if (fi) {
+        fi->bcs_pending = false;             // of this field alone
         flush_for(f);
+        for (cudaEvent_t e : {fi->from_event, fi->done_event})
+            if (e) cudaEventDestroy(e);
         dfree(fi->val[0]); dfree(fi->val[1]); dfree(fi->grad); dfree(fi->partials); dfree(fi->staging);
         if (fi->rec) cudaFree(fi->rec);
         delete fi;
@@ -1725,30 +1774,44 @@ static int field_bc(cuMesh* mesh, FvmField* u, unsigned int region_id, int zero_
         set_error(std::string(what) + ": no region " + std::to_string(region_id));
         return 1;
     }
+    for (cudaEvent_t* e : {&fi->from_event, &fi->done_event})
+        if (!*e && !cuda_ok(cudaEventCreateWithFlags(e, cudaEventDisableTiming), what)) return 1;
     // later conditions on a region replace earlier ones; on meshes of more
-    // regions than the table holds each is applied at once
+    // regions than the table holds, and while the caller captures the stream
+    // (the condition belongs into the graph), each is applied at once
     const int n_regions = (int)mi->topo.regions.size();
-    const bool table = n_regions <= kMaxFieldRegions;
+    const int type = zero_grad ? 1 : 0;
+    const float4 val = make_float4(value.x, value.y, value.z, 0.f);
+    const bool captured = capturing();
     FieldBcTable& tb = fi->bcs;
-    const int r = table ? (int)region_id : 0;
-    if (!fi->bcs_pending) {
-        tb = FieldBcTable{};
-        tb.n = table ? n_regions : 1;
-        for (int k = 0; k < tb.n; ++k) tb.type[k] = -1;
-        for (int k = 0; table && k <= n_regions; ++k) tb.start[k] = mi->num.region_start[k];
+    if (n_regions <= kMaxFieldRegions && !captured) {
+        if (!fi->bcs_pending) {
+            tb = FieldBcTable{};
+            tb.n = n_regions;
+            for (int k = 0; k < n_regions; ++k) tb.type[k] = -1;
+            for (int k = 0; k <= n_regions; ++k) tb.start[k] = mi->num.region_start[k];
+            if (!cuda_ok(cudaEventRecord(fi->from_event, t_stream), what)) return 1;
+        }
+        tb.type[region_id] = type;
+        tb.value[region_id] = val;
+        fi->bcs_pending = true;
+        return 0;
     }
-    tb.type[r] = zero_grad ? 1 : 0;
-    tb.value[r] = make_float4(value.x, value.y, value.z, 0.f);
-    fi->bcs_pending = true;
-    if (table) return 0;
+    if (!flush_field_bcs(mesh, u)) return 1;
     // one region of many: the ghosts before it have no condition, those after it neither
+    tb = FieldBcTable{};
     tb.n = 3;
     tb.start[0] = (uint32_t)mi->dev.N;
     tb.start[1] = mi->num.region_start[region_id];
     tb.start[2] = mi->num.region_start[region_id + 1];
-    tb.type[1] = tb.type[0];
-    tb.value[1] = tb.value[0];
     tb.type[0] = tb.type[2] = -1;
+    tb.type[1] = type;
+    tb.value[1] = val;
+    if (captured) {
+        launch_field_bc(mi->dev, fi->comps, tb, fi->cur, fi->val[0], fi->val[1], t_stream);
+        return launch_ok(what) ? 0 : 1;
+    }
+    fi->bcs_pending = true;
     return flush_field_bcs(mesh, u) ? 0 : 1;
 }
 

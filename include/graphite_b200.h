@@ -518,7 +518,9 @@ int gbFvmApply(cuMesh* mesh, int op, FvmField* u, FvmField* phi, gb_vector phi_c
  *   (fvmScalarBcZeroGrad / fvmVectorBcZeroGrad, src/fvmops.cu:326-366).
  * A field's conditions are recorded and applied together, in one kernel, by
  * the next call that reads or writes the field, with the results of applying
- * each at once (a later condition on a region replaces an earlier one).
+ * each at once (a later condition on a region replaces an earlier one; a
+ * stream that the caller ordered behind the call sees them, and so does a
+ * graph that the call is captured into).
  * Returns 0, or 1 with gbGetLastError() set (unknown region included). */
 int gbFieldInit(cuMesh* mesh, FvmField* u, gb_vector value);
 int gbFieldBcFixed(cuMesh* mesh, FvmField* u, gb_vector value, unsigned int region_id);
