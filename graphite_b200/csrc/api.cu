@@ -166,7 +166,8 @@ struct FieldImpl {
     bool bcs_pending = false;
     // What a caller ordered against the calls that asked for them stays ordered
     // against the launch: from_event is recorded when the first one is asked
-    // for, done_event behind the launch on done_stream (valid: done)
+    // for, done_event behind the launch on done_stream (valid: done), and behind
+    // what a run leaves queued when it returns
     cudaEvent_t from_event = nullptr, done_event = nullptr;
     cudaStream_t done_stream = nullptr;
     bool done = false;
@@ -383,8 +384,8 @@ struct OutsideCapture {
 };
 
 // Applies the field's pending conditions, if any, and orders the thread's
-// stream behind the last application: it may have been launched on another
-// stream, later than the call that asked for it.
+// stream behind the last application (or the end of the last run) on another
+// stream, which may be later than anything the caller knows of.
 bool flush_field_bcs(cuMesh* mesh, FvmField* f) {
     const char* what = "field boundary conditions";
     FieldImpl* fi = impl(f);
@@ -414,6 +415,20 @@ bool flush_field_bcs(cuMesh* mesh, FvmField* f) {
     fi->done_stream = t_stream;
     fi->done = true;
     return launch_ok(what) && cuda_ok(cudaEventRecord(fi->done_event, t_stream), what);
+}
+
+// The runs return with their last kernels still queued; a caller that has waited
+// for the run on the host goes on with other streams.  Those wait then.
+bool leave_queued(FvmField* const* fields, int n, const char* what) {
+    for (int k = 0; k < n; ++k) {
+        FieldImpl* fi = impl(fields[k]);
+        if (!fi->done_event && !cuda_ok(cudaEventCreateWithFlags(&fi->done_event, cudaEventDisableTiming), what))
+            return false;
+        if (!cuda_ok(cudaEventRecord(fi->done_event, t_stream), what)) return false;
+        fi->done_stream = t_stream;
+        fi->done = true;
+    }
+    return true;
 }
 
 // Binds a field's device storage to a mesh's cell order (first use).  Every
@@ -1335,7 +1350,8 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
                 // face states
                 launch_bc_table(mi->dev, a.ghosts, 1 - cur, s);
                 launch_grad_lim(mi->dev, state_of(rho, rhou, rhoe, 1 - cur), grad_of(rho, rhou, rhoe, false), transposed, s);
-                if (!launch_ok("gbEulerRun")) return -1;
+                FvmField* const fields[3] = {rho, rhou, rhoe};
+                if (!launch_ok("gbEulerRun") || !leave_queued(fields, 3, "gbEulerRun")) return -1;
             }
             impl(rho)->cur = impl(rhou)->cur = impl(rhoe)->cur = cur;
             ei->partials_valid = end.finished;   // else the residual is the sum of the field as it is
@@ -1382,7 +1398,8 @@ static int64_t euler_run(cuMesh* mesh, FvmField* rho, FvmField* rhou, FvmField* 
         // the ghost states of the last gradient pass, from the state it read
         // (the buffer before the last update), into both value buffers
         launch_bc_table(mi->dev, gbt, 1 - cur, s);
-        if (!launch_ok("gbEulerRun")) return -1;
+        FvmField* const fields[3] = {rho, rhou, rhoe};
+        if (!launch_ok("gbEulerRun") || !leave_queued(fields, 3, "gbEulerRun")) return -1;
     }
     impl(rho)->cur = impl(rhou)->cur = impl(rhoe)->cur = cur;
     ei->partials_valid = end.finished;   // else the residual is the sum of the field as it is
@@ -1668,7 +1685,8 @@ int64_t gbNSIRun(cuMesh* mesh, FvmField* velocity, FvmField* pressure, FvmField*
                 launch_nsi_grad(mi->dev, (const float*)impl(pressure)->val[1 - cur],
                                 (const float4*)impl(velocity)->val[1 - cur], impl(pressure)->grad, impl(velocity)->grad,
                                 t_nsi.limited, s);
-                if (!launch_ok("gbNSIRun")) return -1;
+                FvmField* const fields[2] = {velocity, pressure};
+                if (!launch_ok("gbNSIRun") || !leave_queued(fields, 2, "gbNSIRun")) return -1;
             }
             impl(velocity)->cur = impl(pressure)->cur = cur;
             ei->partials_valid = end.finished;   // else the residual is the sum of the field as it is
