@@ -54,9 +54,12 @@ constexpr int64_t kLoopNever = int64_t(1) << 62;
 //   WIDE    12,000 to 66,000: layers 11..20 / 19..23, stacked 13..18 / 19..22,
 //           tets 10..14 / 19..21, pyramids 13..18 / 19..21, hexes 18..22 / 23, mixes
 //           18 / 21 at 12,000, 22.6 / 23.0 at 46,000, 24.2 / 23.1 at 54,000.  A launch
-//           of 4 breaks even up to 19,000 cells and for tets, of 8 for 5 faces (16
-//           on the largest with prisms under tets) and one-layer hexes, of 16 for
-//           other hexes.
+//           of 4 breaks even for tets, up to 19,000 cells with 5 faces and up to
+//           57,000 (us per call of 5: 132 / 154 at 50,000) in one layer of prisms,
+//           of 6 on larger layers and stacked prisms, of 8 on the largest of these,
+//           one-layer hexes and small hexes and mixes, of 16 on other hexes.  In a
+//           batch, whose kernels take a launch more, a little earlier (of 6, 12,000
+//           hexes: 169 / 184).
 //   NARROW  layers 14..32 / 22..33, stacked 19..27 / 21..27 (a launch of 8 breaks even
 //           on a layer of prisms, of 16 of hexes and below 94,000 stacked cells, of
 //           32 above), tets 90,000 21.3 / 23.1 (in a batch 24.2 / 23.0), 105,000
@@ -67,11 +70,17 @@ constexpr int64_t kLoopNever = int64_t(1) << 62;
 //           30..35 / 25..27, mixes 42..48 / 27..31.
 constexpr int64_t loop_shortest(LoopForm form, int max_faces, int threads, float sectors, bool batch, int64_t n_iter) {
     if (form == LoopForm::kWide) {
-        if (max_faces <= 4 || (max_faces == 5 && threads <= 64)) return 4;
-        if (max_faces == 5) return sectors <= kLoopStacked || threads <= 192 ? 8 : 16;
+        const bool small = threads <= 64, medium = threads <= 192;
+        if (max_faces <= 4 || (max_faces == 5 && small)) return 4;
+        if (max_faces == 5) {
+            if (sectors <= kLoopLayer) return medium ? 4 : 6;
+            if (sectors <= kLoopStacked) return medium ? 6 : 8;
+            return medium ? 8 : 16;
+        }
         if (sectors <= kLoopLayer) return 8;
-        if (sectors <= kLoopScattered || batch) return 16;
-        return threads <= 160 ? 32 : kLoopNever;
+        if (batch) return sectors <= kLoopScattered ? (small ? 4 : 8) : (small ? 6 : 16);
+        if (small) return 8;
+        return sectors <= kLoopScattered ? 16 : threads <= 160 ? 32 : kLoopNever;
     }
     if (form == LoopForm::kNarrow) {
         if (sectors <= kLoopLayer) return max_faces <= 5 ? 8 : 16;

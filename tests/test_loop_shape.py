@@ -95,10 +95,12 @@ def test_every_shape_gets_the_first_form_that_fits(tmp_path):
 @pytest.mark.parametrize("case,want", [
     ((4, 64, 103, 1000), [4, 4, 4, 4, 4]), ((4, 256, 110, 1000), [4, 4, 4, 4, 4]), ((4, 352, 110, 1000), [8, -1, 8, 8, -1]),
     ((4, 384, 110, 1000), [-1, -1, 8, 8, -1]), ((4, 512, 110, 1000), [-1, -1, 16, -1, -1]), ((4, 512, 110, 50), [-1, -1, 16, 16, 16]),
-    ((5, 64, 50, 1000), [4, 4, 4, 4, 4]), ((5, 192, 91, 1000), [8, 8, 4, 4, 4]), ((5, 256, 50, 1000), [8, 8, 4, 4, 4]),
+    ((5, 64, 50, 1000), [4, 4, 4, 4, 4]), ((5, 192, 50, 1000), [4, 4, 4, 4, 4]), ((5, 224, 50, 1000), [6, 6, 4, 4, 4]),
+    ((5, 192, 91, 1000), [6, 6, 4, 4, 4]), ((5, 224, 91, 1000), [8, 8, 4, 4, 4]), ((5, 192, 112, 1000), [8, 8, 4, 4, 4]),
+    ((5, 256, 50, 1000), [8, 8, 4, 4, 4]), ((6, 64, 98, 1000), [8, 4, 4, 4, 4]), ((6, 64, 112, 1000), [8, 6, 4, 4, 4]),
     ((5, 256, 91, 1000), [16, 16, 4, 4, 4]), ((5, 416, 50, 1000), [8, 8, 8, 8, 8]), ((5, 416, 91, 1000), [32, 32, 8, 8, -1]),
     ((5, 416, 112, 1000), [-1, -1, 8, -1, -1]), ((5, 480, 50, 1000), [32, -1, 16, 32, 32]), ((5, 480, 80, 1000), [-1, -1, -1, -1, -1]),
-    ((6, 192, 66, 1000), [8, 8, 4, 4, 4]), ((6, 192, 98, 1000), [16, 16, 4, 4, 4]), ((6, 192, 112, 1000), [-1, 16, 4, 4, 4]),
+    ((6, 192, 66, 1000), [8, 8, 4, 4, 4]), ((6, 192, 98, 1000), [16, 8, 4, 4, 4]), ((6, 192, 112, 1000), [-1, 16, 4, 4, 4]),
     ((6, 256, 66, 1000), [16, 16, 4, 4, 4]), ((6, 352, 98, 1000), [-1, -1, 8, -1, -1]), ((6, 352, 98, 70), [32, -1, 8, -1, -1]),
     ((6, 352, 66, 1000), [16, 16, 8, 24, 24]), ((5, 224, 103, 1000), [16, 16, 4, 4, 4]), ((6, 512, 66, 1000), [32, -1, 16, 32, 32])])
 def test_where_the_loops_are_taken(tmp_path, case, want):
