@@ -91,13 +91,16 @@ def test_condition_inside_a_capture_is_part_of_the_graph(fields):
         assert np.array_equal(v[: f.n], want) and np.array_equal(v[f.ghosts], want[f.inner])
 
 
-def test_condition_before_a_capture_is_applied_outside_the_graph(fields):
+@pytest.mark.parametrize("asked_on", ["same stream", "default stream"])
+def test_condition_before_a_capture_is_applied_outside_the_graph(fields, asked_on):
     import torch
 
     f, s = fields, torch.cuda.Stream()
-    f.on(s)
+    f.on(s if asked_on == "same stream" else None)
     f.axpy()
     f.zero_grad()
+    s.wait_event(torch.cuda.default_stream().record_event())
+    f.on(s)
     g = torch.cuda.CUDAGraph()
     with torch.cuda.graph(g, stream=s):
         f.gradient()                     # the first use of the field since
@@ -114,12 +117,15 @@ def test_condition_before_a_capture_is_applied_outside_the_graph(fields):
     assert np.all(v[f.ghosts] == 1000.0)      # the replay does not repeat the condition
 
 
+@pytest.mark.parametrize("asked_on", ["stream", "default stream"])
 @pytest.mark.parametrize("first_use", ["asking stream", "other stream"])
-def test_streams_ordered_behind_the_call_see_the_condition(fields, first_use):
+def test_streams_ordered_behind_the_call_see_the_condition(fields, first_use, asked_on):
     import torch
 
     f = fields
     a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    if asked_on == "default stream":
+        a = torch.cuda.default_stream()
     f.on(a)
     f.fixed(500.0)
     after = a.record_event()
@@ -133,12 +139,15 @@ def test_streams_ordered_behind_the_call_see_the_condition(fields, first_use):
     assert np.all(f.values()[f.ghosts] == 500.0)
 
 
-def test_both_streams_in_turn_and_a_capture_of_the_second(fields):
+@pytest.mark.parametrize("asked_on", ["stream", "default stream"])
+def test_both_streams_in_turn_and_a_capture_of_the_second(fields, asked_on):
     """An application on another stream is waited for by a captured use of the field too."""
     import torch
 
     f = fields
     a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    if asked_on == "default stream":
+        a = torch.cuda.default_stream()
     f.on(a)
     f.fixed(500.0)
     b.wait_event(a.record_event())
