@@ -43,8 +43,8 @@ constexpr LoopForm loop_form(int max_faces, int threads) {
 // a warp share the 32-byte sectors of their neighbours' records: `sectors`,
 // counted over a warp's face slots (neighbour_sectors).  One-layer meshes have
 // 50 to 67, prisms stacked in layers 75 to 92, 3-D hexes 97 to 99, prisms under
-// tets, tets, pyramids and mixes of elements 102 to 120.  The narrow forms, with
-// one face in flight, are bound by these loads; WIDE is not.
+// tets, tets, pyramids and mixes of elements 102 to 120.  The narrow forms wait
+// for these loads one face after another; WIDE has them all in flight.
 constexpr float kLoopLayer = 72.f, kLoopStacked = 94.f, kLoopScattered = 105.f;
 constexpr int64_t kLoopNever = int64_t(1) << 62;
 
